@@ -131,8 +131,9 @@ void slime_b200_set_engine(int32_t mode, int32_t band_min_threshold);
 /* The automatic engine rule as 6, 8 or 12 numbers: {band_min_threshold, band_min_periods,
  * band_fast_threshold, band_fast_periods, indep_min_threshold, indep_min_centres,
  * exact_below_threshold, exact_min_centres, grouped_min_threshold, grouped_min_width,
- * grouped_max_width, exact_wide_below_threshold}. Areas 4 x 2^17 chunks wide or more use the
- * exact counts below the larger of exact_below_threshold and exact_wide_below_threshold. Thresholds below exact_below_threshold on areas of
+ * grouped_max_width, exact_wide_below_threshold}. Thresholds below exact_below_threshold (on areas
+ * 4 x 2^17 chunks wide or more: below exact_wide_below_threshold; narrower areas that the grouped
+ * bands take are left to them) on areas of
  * exact_min_centres centres or more use the band engines with bit-sliced exact counts (shared LCG
  * on areas band_fast_periods x 2^17 chunks wide, grouped bands from 4 x 2^17 up to
  * grouped_max_width, else independent bands) while the expected
@@ -150,8 +151,7 @@ void slime_b200_set_engine(int32_t mode, int32_t band_min_threshold);
 int32_t slime_b200_set_engine_rule(const int64_t* rule, int32_t n);
 int32_t slime_b200_get_engine_rule(int64_t* rule, int32_t n);
 
-/* Generator variant of the band engine (results are identical): band_mad_add != 0 issues the
- * per-band add on the multiply pipe instead of the integer ALU. */
+/* Generator variant of earlier versions; accepted and without effect (results never depended on it). */
 void slime_b200_set_tuning(int32_t band_mad_add);
 
 /* Polls of the band kernels' bounded mbarrier waits (row-term bulk copies) before a CTA gives up:

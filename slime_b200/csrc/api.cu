@@ -626,10 +626,7 @@ void slime_b200_last_search_stats(double* kernel_ms, int64_t* launches) {
 
 int64_t slime_b200_last_rare_chunks(void) { return ctx().last_rare; }
 
-void slime_b200_set_tuning(int32_t band_mad_add) {
-    std::lock_guard<std::mutex> lock(ctx().mu);
-    ctx().band_mad_add = band_mad_add ? 1 : 0;
-}
+void slime_b200_set_tuning(int32_t band_mad_add) { (void)band_mad_add; }
 
 int64_t slime_b200_set_wait_limit(int64_t polls) {
     std::lock_guard<std::mutex> lock(ctx().mu);

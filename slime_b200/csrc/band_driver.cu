@@ -17,7 +17,8 @@ constexpr uint32_t kRareCap = 1u << 20;
 
 bool Context::ensure_band() {
     if (band_ready) return true;
-    cudaError_t e = band_prepare();
+    cudaError_t e = column_prepare();
+    if (e == cudaSuccess) e = plane_prepare();
     if (e != cudaSuccess) { set_error("band smem", e); return false; }
     std::vector<uint64_t> t;
     std::vector<uint32_t> o;
@@ -41,11 +42,12 @@ bool Context::ensure_band() {
 int32_t Context::engine_for(const SearchSpec& q) const {
     if (engine_override == 4) return kAlgoBandExact;
     if (engine_override == 5) return kAlgoIndepExact;
-    if (engine_override == 7) return kAlgoGroupedExact;
+    const bool groups_fit = 2 * q.rd_max + 1 <= kGroupedMaxPeriods * kP;  // 16 copies at most
+    if (engine_override == 7) return groups_fit ? kAlgoGroupedExact : kAlgoBandExact;
     if (engine_override == 1 || q.min_size < 28) return kAlgoGeneral;
     if (engine_override == 2) return kAlgoBand;
     if (engine_override == 3) return kAlgoIndep;
-    if (engine_override == 6) return kAlgoGrouped;
+    if (engine_override == 6) return groups_fit ? kAlgoGrouped : kAlgoBand;
     // The rule's numbers are measured crossovers (slime_b200/autotune.py writes them; the
     // defaults are the B200 values). The shared LCG pays off with many periods (its work is
     // shared by every band and phase pair) and a high threshold.
@@ -53,22 +55,20 @@ int32_t Context::engine_for(const SearchSpec& q) const {
     // Low thresholds: exact counts of every centre, while the sites stay few enough to collect
     // (the band engines emit every site in range; the general scan gates by count on the device).
     constexpr double kExactMaxSites = 1e9;
-    const int32_t exact_below =
-        w >= kGroupedExactMinPeriods * kP ? std::max(exact_below_threshold, exact_wide_below_threshold) : exact_below_threshold;
-    if (q.min_size < exact_below && w * w >= exact_min_centres &&
-        (double)w * (double)w * tail_share(q.min_size) <= kExactMaxSites)
-        // Exact counts cost the same per centre in every mode; the generator's sharing decides:
-        // independent bands on narrow areas, grouped bands from 4 periods (measured on B200:
-        // 1.1-1.3 against 1.0 T/s at 4.6-9 periods, 0.9 against 1.0 at 3 periods), the shared
-        // LCG on the widest.
-        return w >= (int64_t)band_fast_periods * kP ? kAlgoBandExact
-               : w >= kGroupedExactMinPeriods * kP && w <= grouped_max_width && w <= kGroupedMaxPeriods * kP
-                   ? kAlgoGroupedExact
-                   : kAlgoIndepExact;
+    const bool wide = w >= kGroupedExactMinPeriods * kP;
+    const bool grouped_width = w >= grouped_min_width && w <= grouped_max_width && w <= kGroupedMaxPeriods * kP;
     // Areas one to several periods wide: X phase pairs with groups of Z period copies.
-    if (q.min_size >= grouped_min_threshold && w >= grouped_min_width && w <= grouped_max_width &&
-        w <= kGroupedMaxPeriods * kP)
-        return kAlgoGrouped;
+    const bool grouped = q.min_size >= grouped_min_threshold && grouped_width;
+    if (!(grouped && !wide) && q.min_size < (wide ? exact_wide_below_threshold : exact_below_threshold) &&
+        w * w >= exact_min_centres && (double)w * (double)w * tail_share(q.min_size) <= kExactMaxSites)
+        // Exact counts cost the same per centre in every mode; the generator's sharing and how full
+        // the words are decide: independent bands on narrow areas, grouped bands from 4 periods
+        // (measured on B200: 1.71 against 1.39 T/s at 4.6 periods, 1.35 against 1.39 at 3 periods), the
+        // shared LCG on the widest.
+        return w >= (int64_t)band_fast_periods * kP ? kAlgoBandExact
+               : wide && w <= grouped_max_width && w <= kGroupedMaxPeriods * kP ? kAlgoGroupedExact
+                                                                                : kAlgoIndepExact;
+    if (grouped) return kAlgoGrouped;
     if ((q.min_size >= band_min_threshold && w >= (int64_t)band_min_periods * kP) ||
         (q.min_size >= band_fast_threshold && w >= (int64_t)band_fast_periods * kP))
         return kAlgoBand;
@@ -76,48 +76,94 @@ int32_t Context::engine_for(const SearchSpec& q) const {
     return kAlgoGeneral;
 }
 
-BandGeom band_geometry(int64_t W, int64_t H, int mode, int sm_count) {
+BandGeom band_geometry(int64_t W, int64_t H, int mode, bool planes, int sm_count) {
     BandGeom g{};
     const bool indep = mode == kBandIndep, grouped = mode == kBandGrouped;
     g.indep = indep;
+    g.planes = planes;
     g.transposed = mode == kBandShared && W < 2 * kP && H >= 2 * kP;
     g.width_u = g.transposed ? H : W;
     g.height_v = g.transposed ? W : H;
-    const int out_w = band_tile_out_w();
+    const int out_w = planes ? plane_tile_out_w(mode) : column_tile_out_w();
     const int nb_max = band_max_bands();
-    // Shared LCG: X phases and Z bands 2^17 apart. Independent bands: one phase, nJ bands of
-    // `stride` rows each (at least 256 rows a band, at most 32 bands). Grouped bands: X phase
-    // pairs and G groups of `copies` bands 2^17 apart (G a power of two, G * copies <= 16), group
-    // g starting at row g * stride with G * stride = 2^17 (or the whole height in one copy).
+    // Shared LCG: X phases and Z bands 2^17 apart. Independent bands: one phase, 32 bands (one a bit;
+    // fewer only below 8 rows a band) of `stride` rows each. Grouped bands: X phase pairs and G groups
+    // of `copies` bands 2^17 apart (G * copies <= 16), group g starting at row g * stride, where
+    // G * stride covers 2^17 (or the whole height in one copy). The plane kernels take as many groups
+    // as fit (each fills bits of a word); the column kernels want G a power of two.
     g.nI = indep ? 1 : (g.width_u + kP - 1) / kP;
     if (grouped) {
         const int64_t copies = std::max<int64_t>(1, (g.height_v + kP - 1) / kP);
-        int64_t G = kGroupedMaxBands;
-        while (G > 1 && G * copies > kGroupedMaxBands) G >>= 1;
+        int64_t G = std::max<int64_t>(1, kGroupedMaxBands / copies);
+        if (!planes)
+            while (G & (G - 1)) --G;
         g.groups = (int32_t)G;
         g.nJ = G * copies;
-        g.stride = copies > 1 ? kP / G : (g.height_v + G - 1) / G;
+        g.stride = ((copies > 1 ? kP : g.height_v) + G - 1) / G;
     } else {
-        g.nJ = indep ? std::max<int64_t>(1, std::min<int64_t>(nb_max, g.height_v / 256)) : (g.height_v + kP - 1) / kP;
+        g.nJ = indep ? std::max<int64_t>(1, std::min<int64_t>(nb_max, g.height_v / 8)) : (g.height_v + kP - 1) / kP;
         g.stride = indep ? (g.height_v + g.nJ - 1) / g.nJ : kP;
     }
     g.ubase = (int32_t)(indep ? g.width_u : std::min(kP, g.width_u));
     g.vbase = (int32_t)std::min(g.stride, g.height_v);
     g.vrows = g.vbase + 16;
-    g.vrows_alloc = g.vbase + 32;  // zero rows: 8-row bulk copies never run past the end
+    g.vrows_alloc = g.vbase + 32;  // zero rows: the bulk copies of a batch never run past the end
     g.ngroups = (g.nJ + nb_max - 1) / nb_max;
     g.u_tiles = (g.ubase + out_w - 1) / out_w;
-    g.band_h = (int32_t)std::min<int64_t>(2048, std::max<int64_t>(256, g.vbase));
-    if (indep) {
-        // Enough tiles for two waves of CTAs where the area allows it, tiles of 64+ rows.
-        const int64_t want = (2 * (int64_t)sm_count + g.u_tiles - 1) / g.u_tiles;
-        const int64_t vt = std::max<int64_t>((g.vbase + 2047) / 2048, std::min<int64_t>((g.vbase + 63) / 64, want));
-        g.band_h = (int32_t)((g.vbase + vt - 1) / vt);
-    }
-    g.v_tiles = (g.vbase + g.band_h - 1) / g.band_h;
     g.pairs = (g.nI + 1) / 2;
+    // Tile height: the tiles of a launch run in waves of `slots` CTAs, each tile 16 halo rows taller
+    // than its centres. The height (at most 2,048 rows) whose waves take the fewest rows wins; with
+    // many waves the last one hardly counts. (Radius 20,011, 40 columns of tiles: 8 tiles high made
+    // 320 tiles on 148 CTAs, 3 waves of 173 rows where 7 make 2 of 195.)
+    const int64_t slots = band_grid(planes, sm_count), columns = g.u_tiles * g.pairs;
+    int64_t best_vt = 0;
+    double best_rows = 0;
+    for (int64_t vt = (g.vbase + 2047) / 2048; vt <= std::max<int64_t>(1, (g.vbase + 7) / 8); ++vt) {
+        const int64_t h = (g.vbase + vt - 1) / vt, tiles = columns * ((g.vbase + h - 1) / h);
+        const double waves = tiles > 16 * slots ? (double)tiles / (double)slots + 0.5
+                                                : (double)((tiles + slots - 1) / slots);
+        const double rows = waves * (double)(h + 16 + 8);  // and a batch's worth of set-up
+        if (!best_vt || rows < best_rows) {
+            best_vt = vt;
+            best_rows = rows;
+        }
+        if (tiles > 24 * slots) break;
+    }
+    g.band_h = (int32_t)((g.vbase + best_vt - 1) / best_vt);
+    g.v_tiles = (g.vbase + g.band_h - 1) / g.band_h;
     g.tiles = g.u_tiles * g.v_tiles * g.pairs;
     return g;
+}
+
+int band_grid(bool planes, int sm_count) { return sm_count * (planes ? plane_ctas_per_sm() : 1); }
+
+size_t band_row_table_words(const BandGeom& g) {
+    const int mode = g.indep ? kBandIndep : g.groups > 0 ? kBandGrouped : kBandShared;
+    return (size_t)g.ngroups * g.vrows_alloc * (g.planes ? plane_row_words(mode) : column_row_words(mode));
+}
+
+cudaError_t launch_band_terms(uint64_t* ct, uint32_t* rt, const BandGeom& g, int64_t seed, int32_t area_x0,
+                              int32_t area_z0, cudaStream_t s) {
+    // Columns carry no seed; rows carry it. Transposed searches swap which axis is x.
+    const int32_t col_first = (g.transposed ? area_z0 : area_x0) - 8;
+    const int32_t row_first = (g.transposed ? area_x0 : area_z0) - 8;
+    const cudaError_t e = launch_column_terms(ct, col_first, (int32_t)(g.width_u + 16), g.transposed, s);
+    if (e != cudaSuccess) return e;
+    return g.planes ? launch_plane_row_terms(rt, g.vrows_alloc, g.vrows, (int32_t)g.nJ, row_first, g.height_v + 16, g.stride,
+                                             seed, g.transposed, g.indep, g.groups, s)
+                    : launch_column_row_terms(rt, g.vrows_alloc, g.vrows, (int32_t)g.nJ, row_first, g.height_v + 16,
+                                              g.stride, seed, g.transposed, g.groups, s);
+}
+
+cudaError_t launch_band_scan(const BandArgs& a, int grid, cudaStream_t s) {
+    return band_planes(band_mode(a), a.exact != 0) ? launch_plane_scan(a, grid, s) : launch_column_scan(a, grid, s);
+}
+
+// 0..3: columns in words, by mode (shared, grouped) and survivor lists; 4..7: bit planes.
+int band_class(const BandArgs& a) {
+    const int mode = band_mode(a);
+    if (band_planes(mode, a.exact != 0)) return mode == kBandIndep ? 4 + (a.exact ? 1 : 0) : mode == kBandGrouped ? 6 : 7;
+    return (mode == kBandGrouped ? 2 : 0) + (band_keeps_candidates(a.min_size) ? 1 : 0);
 }
 
 bool Context::scan_band(const SearchSpec& q, std::vector<Hit>& best, std::vector<uint32_t>& h,
@@ -126,28 +172,24 @@ bool Context::scan_band(const SearchSpec& q, std::vector<Hit>& best, std::vector
     const int64_t W = 2 * q.rd_max + 1, H = W;
     const int32_t area_x0 = (int32_t)((int64_t)q.center_x - q.rd_max);
     const int32_t area_z0 = (int32_t)((int64_t)q.center_z - q.rd_max);
-    const BandGeom G = band_geometry(W, H, mode, sm_count);
-    const bool indep = G.indep, split = G.indep || G.groups > 0;
+    const BandGeom G = band_geometry(W, H, mode, band_planes(mode, exact), sm_count);
+    const bool indep = G.indep;
     const bool transposed = G.transposed;
     const int64_t width_u = G.width_u, height_v = G.height_v;
     const int nb_max = band_max_bands();
     const int64_t nJ = G.nJ, stride = G.stride;
-    const int32_t ubase = G.ubase, vbase = G.vbase, vrows = G.vrows, vrows_alloc = G.vrows_alloc;
+    const int32_t ubase = G.ubase, vbase = G.vbase, vrows = G.vrows;
     const int64_t ngroups = G.ngroups;
     cudaError_t e;
     if ((e = xt.reserve((size_t)width_u + 16)) != cudaSuccess ||
-        (e = rt.reserve((size_t)ngroups * vrows_alloc * band_row_words(split))) != cudaSuccess ||
+        (e = rt.reserve(band_row_table_words(G))) != cudaSuccess ||
         (e = counters.reserve(4)) != cudaSuccess ||
         (e = hits.reserve(hit_capacity(q.max_results))) != cudaSuccess ||
         (e = fixed.reserve(1u << 20)) != cudaSuccess) {
         set_error("alloc", e);
         return false;
     }
-    const int32_t col_first = (transposed ? area_z0 : area_x0) - 8;
-    const int32_t row_first = (transposed ? area_x0 : area_z0) - 8;
-    if ((e = launch_band_terms(xt.ptr, col_first, (int32_t)(width_u + 16), rt.ptr, vrows_alloc, vrows,
-                               (int32_t)nJ, row_first, height_v + 16, stride, q.seed, transposed, indep, G.groups,
-                               stream)) != cudaSuccess) {
+    if ((e = launch_band_terms(xt.ptr, rt.ptr, G, q.seed, area_x0, area_z0, stream)) != cudaSuccess) {
         set_error("band terms", e);
         return false;
     }
@@ -185,7 +227,7 @@ bool Context::scan_band(const SearchSpec& q, std::vector<Hit>& best, std::vector
 
     const int64_t u_tiles = G.u_tiles, v_tiles = G.v_tiles;
     const int32_t band_h = G.band_h;
-    const int grid = sm_count;
+    const int grid = band_grid(G.planes, sm_count);
     const uint64_t cap = hits.count;
     // Count histogram on the device (first-draw counts of every centre in range, corrected for
     // rare chunks by the fix-up) and an emission gate: only centres whose count reaches emit_min
@@ -221,7 +263,7 @@ bool Context::scan_band(const SearchSpec& q, std::vector<Hit>& best, std::vector
                 BandArgs a{};
                 a.ct = xt.ptr;
                 a.ncols = width_u + 16;
-                a.rt = rt.ptr + (size_t)g * vrows_alloc * band_row_words(split);
+                a.rt = rt.ptr + (size_t)g * (band_row_table_words(G) / (size_t)ngroups);
                 a.vrows = vrows;
                 a.vbase = vbase;
                 a.ubase = ubase;
@@ -246,11 +288,10 @@ bool Context::scan_band(const SearchSpec& q, std::vector<Hit>& best, std::vector
                 a.cap = cap;
                 a.emitted = counters.ptr;
                 a.overflow = flags.ptr;
-                a.one = 1u;
-                a.mad_add = band_mad_add;
                 a.indep = indep ? 1 : 0;
                 a.groups = G.groups;
                 a.exact = exact ? 1 : 0;
+                a.one = 1u;
                 a.poll_limit = wait_polls;
                 a.hist = dhist;
                 a.emit_min = emit_min;
@@ -368,9 +409,8 @@ bool Context::scan_band(const SearchSpec& q, std::vector<Hit>& best, std::vector
             return false;
         }
         if (*(uint32_t*)pinned & 4u) { set_error("band engine: row-term copy timed out", cudaErrorLaunchTimeout); return false; }
-        if ((*(uint32_t*)pinned & 1u) && !exact) {
+        if (*(uint32_t*)pinned & 1u) {
             // A 4-row strip too dense for the byte-lane box: redo the search with the general scan.
-            band_fallbacks++;
             std::fill(h.begin(), h.end(), 0u);
             best.clear();
             return scan_general(q, best, h, cancelled);

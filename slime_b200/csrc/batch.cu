@@ -51,7 +51,7 @@ constexpr uint64_t kHitCapMax = 16ull << 20;    // per search; larger searches r
 }  // namespace
 
 cudaError_t run_band_items(std::vector<BandArgs>& items, BandArgs* args_dev, int64_t* prefix_dev,
-                           unsigned long long* heads_dev, int grid, cudaStream_t s, int64_t* launches) {
+                           unsigned long long* heads_dev, int sm_count, cudaStream_t s, int64_t* launches) {
     const size_t m = items.size();
     if (m == 0) return cudaSuccess;
     std::stable_sort(items.begin(), items.end(),
@@ -64,12 +64,16 @@ cudaError_t run_band_items(std::vector<BandArgs>& items, BandArgs* args_dev, int
         (e = cudaMemsetAsync(heads_dev, 0, kBandClasses * sizeof(unsigned long long), s)) != cudaSuccess)
         return e;
     for (size_t i0 = 0; i0 < m;) {
-        const int cls = band_class(items[i0]);
+        const int cls = band_class(items[i0]), mode = band_mode(items[i0]);
+        const bool planes = band_planes(mode, items[i0].exact != 0);
         size_t i1 = i0 + 1;
         while (i1 < m && band_class(items[i1]) == cls) ++i1;
-        if ((e = launch_band_batch(args_dev + i0, prefix_dev + i0, (int32_t)(i1 - i0), heads_dev + cls, cls, grid, s)) !=
-            cudaSuccess)
-            return e;
+        const int grid = band_grid(planes, sm_count);
+        const int32_t n = (int32_t)(i1 - i0);
+        e = planes ? launch_plane_batch(args_dev + i0, prefix_dev + i0, n, heads_dev + cls, mode, items[i0].exact != 0, grid, s)
+                   : launch_column_batch(args_dev + i0, prefix_dev + i0, n, heads_dev + cls, mode,
+                                         band_keeps_candidates(items[i0].min_size), grid, s);
+        if (e != cudaSuccess) return e;
         if (launches) ++*launches;
         i0 = i1;
     }
@@ -167,7 +171,8 @@ int32_t Context::search_batch(const SearchSpec* reqs, int32_t n, ExtChunkResult*
         p.idx = i;
         p.exact = exact;
         const int64_t W = 2 * q.rd_max + 1;
-        p.g = band_geometry(W, W, algo == kAlgoGeneral ? kBandIndep : band_mode_of(algo), sm_count);
+        const int mode = algo == kAlgoGeneral ? kBandIndep : band_mode_of(algo);
+        p.g = band_geometry(W, W, mode, band_planes(mode, exact), sm_count);
         p.area_x0 = (int32_t)((int64_t)q.center_x - q.rd_max);
         p.area_z0 = (int32_t)((int64_t)q.center_z - q.rd_max);
         const double centres = (double)W * (double)W;
@@ -184,7 +189,7 @@ int32_t Context::search_batch(const SearchSpec* reqs, int32_t n, ExtChunkResult*
         p.hit_off = hit_total;
         p.rare_off = rare_total;
         ct_total += (size_t)p.g.width_u + 16;
-        rt_total += (size_t)p.g.ngroups * p.g.vrows_alloc * band_row_words(p.g.indep || p.g.groups > 0);
+        rt_total += band_row_table_words(p.g);
         hit_total += p.hit_cap;
         rare_total += p.rare_cap;
         plan.push_back(p);
@@ -241,9 +246,8 @@ int32_t Context::search_batch(const SearchSpec* reqs, int32_t n, ExtChunkResult*
             a.cap = p.hit_cap;
             a.emitted = bt_counts.ptr + 2 * s;
             a.overflow = bt_flags.ptr + 4 * s;
-            a.one = 1u;
-            a.mad_add = band_mad_add;
             a.exact = p.exact ? 1 : 0;
+            a.one = 1u;
             a.poll_limit = wait_polls;
             a.indep = g.indep ? 1 : 0;
             a.groups = g.groups;
@@ -259,11 +263,8 @@ int32_t Context::search_batch(const SearchSpec* reqs, int32_t n, ExtChunkResult*
             const SearchSpec& q = reqs[p.idx];
             const BandGeom& g = p.g;
             const int64_t W = 2 * q.rd_max + 1;
-            const int32_t col_first = (g.transposed ? p.area_z0 : p.area_x0) - 8;
-            const int32_t row_first = (g.transposed ? p.area_x0 : p.area_z0) - 8;
-            if ((e = launch_band_terms(bt_ct.ptr + p.ct_off, col_first, (int32_t)(g.width_u + 16), bt_rt.ptr + p.rt_off,
-                                       g.vrows_alloc, g.vrows, (int32_t)g.nJ, row_first, g.height_v + 16,
-                                       g.stride, q.seed, g.transposed, g.indep, g.groups, stream)) != cudaSuccess ||
+            if ((e = launch_band_terms(bt_ct.ptr + p.ct_off, bt_rt.ptr + p.rt_off, g, q.seed, p.area_x0, p.area_z0, stream)) !=
+                    cudaSuccess ||
                 (e = launch_rare_scan(rare_targets.ptr, rare_offsets.ptr, q.seed, p.area_z0 - 8, (int32_t)(W + 16),
                                       p.area_x0 - 8, (int32_t)(W + 16), bt_rare.ptr + p.rare_off, p.rare_cap,
                                       bt_flags.ptr + 4 * s + 2, stream)) != cudaSuccess) {

@@ -151,20 +151,19 @@ struct Context {
     int64_t indep_min_centres = 400040001;
     // Below exact_below_threshold, areas of exact_min_centres centres or more use the band engines
     // with bit-sliced exact counts (shared LCG on areas band_fast_periods periods wide, else
-    // independent bands), as long as the expected number of sites stays below kExactMaxSites.
-    int32_t exact_below_threshold = 45;
+    // independent bands), as long as the expected number of sites stays below kExactMaxSites and the
+    // grouped bands do not take them.
+    int32_t exact_below_threshold = 51;
     int64_t exact_min_centres = 400040001;
     // Grouped bands for areas grouped_min_width .. grouped_max_width chunks wide (at most
     // kGroupedMaxPeriods periods) from grouped_min_threshold, before the shared-LCG rule.
-    int32_t grouped_min_threshold = 46;
+    int32_t grouped_min_threshold = 48;
     // Areas kGroupedExactMinPeriods periods wide or more use exact counts below this threshold
     // instead (their exact modes share more of the generator's work).
-    int32_t exact_wide_below_threshold = 45;
-    int64_t grouped_min_width = 200001;
+    int32_t exact_wide_below_threshold = 48;
+    int64_t grouped_min_width = 300001;
     int64_t grouped_max_width = 2000001;
     int64_t last_rare = 0;             // rare redraw chunks found by the last band search
-    int64_t band_fallbacks = 0;        // band searches redone by the general scan
-    int32_t band_mad_add = 1;          // generator variant: band adds on the multiply pipe
     uint32_t wait_polls = 1u << 22;    // bounded mbarrier waits of the band kernels
 
     // Y-scan configuration (set_y_scan_config) and the tables built from it.

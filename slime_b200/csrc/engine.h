@@ -85,23 +85,22 @@ struct BandArgs {
     uint64_t cap;
     unsigned long long* emitted;
     unsigned int* overflow;
-    uint32_t one;            // the value 1 (run time): band adds as multiply-adds when mad_add
-    int32_t mad_add;
     int32_t indep;           // 1: independent bands (no shared LCG work, one X phase)
     int32_t exact;           // 1: bit-sliced exact counts of every centre (no bounds)
+    uint32_t one;            // the value 1 (run time): keeps band adds on the multiply pipe
     uint32_t poll_limit;     // polls of a row-term mbarrier before the CTA gives up (bit 4 of overflow)
     unsigned int* hist;      // if set: kHistBins counters of every centre in range, by count
     int32_t emit_min;        // centres in range are appended to `out` only from this count on
     int64_t row_stride;      // input rows between band j and band j + 1 (2^17 with the shared LCG;
                              // grouped bands: between group g and group g + 1)
-    int32_t groups;          // grouped bands (G > 0): band m = copy * G + group, copies 2^17 apart
+    int32_t groups;          // grouped bands (G > 0): G groups of nb / G copies 2^17 apart
     int32_t pad_;
 };
 
 // Tiling of one band search (band_driver.cu): axes (u = phase axis, v = band axis), phases,
 // bands, base sizes and tiles, as the band kernels expect them.
 struct BandGeom {
-    bool indep, transposed;
+    bool indep, transposed, planes;
     int32_t groups;  // grouped bands: G groups of nJ / G copies (0 otherwise)
     int64_t width_u, height_v, nI, nJ, stride, ngroups;
     int32_t ubase, vbase, vrows, vrows_alloc, band_h;
@@ -109,33 +108,55 @@ struct BandGeom {
 };
 // Band modes of band_geometry.
 constexpr int kBandShared = 0, kBandIndep = 1, kBandGrouped = 2;
-BandGeom band_geometry(int64_t W, int64_t H, int mode, int sm_count);
+// Tiling of a search area; `planes` says which kernels run it (band_planes).
+BandGeom band_geometry(int64_t W, int64_t H, int mode, bool planes, int sm_count);
 
-size_t band_smem_bytes();
-int band_tile_out_w();
+// Two kernel families share BandArgs. scan_band.cu: a word holds 32 columns of one combo (bounded
+// counts of shared and grouped bands). scan_planes.cu: a word holds 32 combos of one column (exact
+// counts, and independent bands).
+inline bool band_planes(int mode, bool exact) { return exact || mode == kBandIndep; }
+inline int band_mode(const BandArgs& a) { return a.indep ? kBandIndep : a.groups ? kBandGrouped : kBandShared; }
 int band_max_bands();
-cudaError_t band_prepare();
+bool band_keeps_candidates(int min_size);
+
+int column_tile_out_w();
+int column_row_words(int mode);
+cudaError_t column_prepare();
+cudaError_t launch_column_scan(const BandArgs& a, int grid, cudaStream_t s);
+cudaError_t launch_column_batch(const BandArgs* args, const int64_t* prefix, int32_t nsearch, unsigned long long* head,
+                                int mode, bool cands, int grid, cudaStream_t s);
+cudaError_t launch_column_row_terms(uint32_t* rt, int32_t vrows_alloc, int32_t vrows, int32_t nj, int32_t row_first,
+                                    int64_t row_limit, int64_t row_stride, int64_t seed, bool transposed, int32_t groups,
+                                    cudaStream_t s);
+cudaError_t launch_column_terms(uint64_t* ct, int32_t first, int32_t n, bool transposed, cudaStream_t s);
+
+int plane_tile_out_w(int mode);
+int plane_row_words(int mode);
+int plane_ctas_per_sm();
+cudaError_t plane_prepare();
+cudaError_t launch_plane_scan(const BandArgs& a, int grid, cudaStream_t s);
+cudaError_t launch_plane_batch(const BandArgs* args, const int64_t* prefix, int32_t nsearch, unsigned long long* head,
+                               int mode, bool exact, int grid, cudaStream_t s);
+cudaError_t launch_plane_row_terms(uint32_t* rt, int32_t vrows_alloc, int32_t vrows, int32_t nj, int32_t row_first,
+                                   int64_t row_limit, int64_t row_stride, int64_t seed, bool transposed, bool indep,
+                                   int32_t groups, cudaStream_t s);
+
+// Column and row terms of a search (W x H centres from area_x0, area_z0) into ct and rt.
+cudaError_t launch_band_terms(uint64_t* ct, uint32_t* rt, const BandGeom& g, int64_t seed, int32_t area_x0,
+                              int32_t area_z0, cudaStream_t s);
+// Words of the row-term table of a search, and the CTAs of a full grid of its kernel.
+size_t band_row_table_words(const BandGeom& g);
+int band_grid(bool planes, int sm_count);
 cudaError_t launch_band_scan(const BandArgs& a, int grid, cudaStream_t s);
-// Tiles of many band searches of one launch class (band_class: band mode, survivor lists, exact
-// counts; kBandClasses of them) in one persistent launch: args[i] (device) describes search i,
-// prefix[i] (device, nsearch + 1 entries, increasing from any start) is its first tile in the
-// launch, *head (device, zeroed) is the tile queue. Item i runs tiles tile_begin .. tile_begin +
-// prefix[i+1] - prefix[i] - 1 of its search (tile_end is unused).
-constexpr int kBandClasses = 9;
+// Launch classes: kernel family, band mode, and survivor lists or exact counts.
+constexpr int kBandClasses = 8;
 int band_class(const BandArgs& a);
-cudaError_t launch_band_batch(const BandArgs* args, const int64_t* prefix, int32_t nsearch,
-                              unsigned long long* head, int cls, int grid, cudaStream_t s);
 // Uploads band work items of any classes (reordered by class in place) and runs them: one
-// persistent launch per class present. args_dev / prefix_dev hold items.size() (+1) entries,
-// heads_dev kBandClasses counters. Adds the launches made to *launches.
+// persistent launch per class present, whose CTAs take the tiles of the class's items from a device
+// counter. args_dev / prefix_dev hold items.size() (+1) entries, heads_dev kBandClasses counters.
+// Item i runs tiles tile_begin .. tile_end - 1 of its search. Adds the launches made to *launches.
 cudaError_t run_band_items(std::vector<BandArgs>& items, BandArgs* args_dev, int64_t* prefix_dev,
-                           unsigned long long* heads_dev, int grid, cudaStream_t s, int64_t* launches);
-// Words of a row-term record: per-band low bits (independent and grouped bands) or shared ones.
-int band_row_words(bool split);
-cudaError_t launch_band_terms(uint64_t* ct, int32_t col_first, int32_t ncols, uint32_t* rt,
-                              int32_t vrows_alloc, int32_t vrows, int32_t nj, int32_t row_first,
-                              int64_t row_limit, int64_t row_stride, int64_t seed, bool transposed,
-                              bool indep, int32_t groups, cudaStream_t s);
+                           unsigned long long* heads_dev, int sm_count, cudaStream_t s, int64_t* launches);
 
 // ---- rare redraw correction (rare_fix.cu) ------------------------------------------------
 

@@ -116,14 +116,14 @@ void plan_job(Job& j, const Context& c) {
         j.bytes = (size_t)(W + 16) * 16 + hit_capacity(q.max_results) * sizeof(Hit);
         return;
     }
-    j.g = band_geometry(W, W, band_mode_of(algo), c.sm_count);
+    j.g = band_geometry(W, W, band_mode_of(algo), band_planes(band_mode_of(algo), j.exact), c.sm_count);
     j.area_x0 = (int32_t)((int64_t)q.center_x - q.rd_max);
     j.area_z0 = (int32_t)((int64_t)q.center_z - q.rd_max);
     j.hit_cap = (uint64_t)std::min<double>((double)(16u << 20), 2.0 * expect + 65536.0);
     const double halo = (double)(W + 16) * (double)(W + 16);
     j.rare_cap = (uint32_t)std::min<double>(1 << 20, 3.0 * halo * rare_share() + 1024.0);
     j.bytes = align256((size_t)(j.g.width_u + 16) * 8) +
-              align256((size_t)j.g.ngroups * j.g.vrows_alloc * band_row_words(j.g.indep || j.g.groups > 0) * 4) +
+              align256(band_row_table_words(j.g) * 4) +
               align256((size_t)j.hit_cap * sizeof(Hit)) + align256((size_t)j.rare_cap * sizeof(int2)) +
               align256(2 * kHistBins * sizeof(unsigned int)) + 256;
 }
@@ -148,7 +148,7 @@ bool Server::start(Job* j) {
     if (e != cudaSuccess) { c.set_error("server alloc", e); j->mem = nullptr; return false; }
     char* p = (char*)j->mem;
     j->ct = (uint64_t*)p; p += align256((size_t)(j->g.width_u + 16) * 8);
-    j->rt = (uint32_t*)p; p += align256((size_t)j->g.ngroups * j->g.vrows_alloc * band_row_words(j->g.indep || j->g.groups > 0) * 4);
+    j->rt = (uint32_t*)p; p += align256(band_row_table_words(j->g) * 4);
     j->hits = (Hit*)p; p += align256((size_t)j->hit_cap * sizeof(Hit));
     j->rare = (int2*)p; p += align256((size_t)j->rare_cap * sizeof(int2));
     j->hist = (unsigned int*)p; p += align256(2 * kHistBins * sizeof(unsigned int));
@@ -157,13 +157,9 @@ bool Server::start(Job* j) {
     const SearchSpec& q = j->q;
     const BandGeom& g = j->g;
     const int64_t W = 2 * q.rd_max + 1;
-    const int32_t col_first = (g.transposed ? j->area_z0 : j->area_x0) - 8;
-    const int32_t row_first = (g.transposed ? j->area_x0 : j->area_z0) - 8;
     if ((e = cudaMemsetAsync(p, 0, 256, c.stream)) != cudaSuccess ||
         (e = cudaMemsetAsync(j->hist, 0, 2 * kHistBins * sizeof(unsigned int), c.stream)) != cudaSuccess ||
-        (e = launch_band_terms(j->ct, col_first, (int32_t)(g.width_u + 16), j->rt, g.vrows_alloc, g.vrows,
-                               (int32_t)g.nJ, row_first, g.height_v + 16, g.stride, q.seed, g.transposed, g.indep,
-                               g.groups, c.stream)) != cudaSuccess ||
+        (e = launch_band_terms(j->ct, j->rt, g, q.seed, j->area_x0, j->area_z0, c.stream)) != cudaSuccess ||
         (e = launch_rare_scan(c.rare_targets.ptr, c.rare_offsets.ptr, q.seed, j->area_z0 - 8, (int32_t)(W + 16),
                               j->area_x0 - 8, (int32_t)(W + 16), j->rare, j->rare_cap, j->flags + 2,
                               c.stream)) != cudaSuccess) {
@@ -368,9 +364,8 @@ bool Server::step(std::vector<Job*>& live) {
         a.cap = j->hit_cap;
         a.emitted = j->counts;
         a.overflow = j->flags;
-        a.one = 1u;
-        a.mad_add = c.band_mad_add;
         a.exact = j->exact ? 1 : 0;
+        a.one = 1u;
         a.poll_limit = c.wait_polls;
         a.indep = g.indep ? 1 : 0;
         a.groups = g.groups;
