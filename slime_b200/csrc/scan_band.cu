@@ -136,6 +136,7 @@ __device__ __forceinline__ uint32_t bytes_at_least(uint32_t v, uint32_t t4) {
 
 struct Tile {
     int u0, v0, i0, out_h;
+    int nb, phases;  // bands and X phases that hold a centre of the area in this tile
 };
 
 // The kGenW words of one plane at dst (16-byte aligned), as uint4 stores.
@@ -387,9 +388,9 @@ __device__ __forceinline__ void second_test(BandSmem& S, const BandArgs& a, cons
 
 // Counts one 4-row strip (rows 4t..4t+3 of ring slot `slot`) for the warp's four combo slots as
 // one straight-line block: 4x4 block counts, 20-column strip sums, rolling 20x20 boxes and the
-// threshold test. Only when a lane flags a group does the warp take the second test. With the
-// shared LCG, slots of combos beyond the launch's band count read zero planes and never flag; grouped
-// bands use two slots per warp (32 combos) and skip combos beyond the band count.
+// threshold test. Only when a lane flags a group does the warp take the second test. Combos without
+// a centre in the tile are skipped (warp-uniform): with 19.07 periods (radius 1,250,000) that leaves
+// 38 of the 64 slots and one phase of the last pair; grouped bands use two slots per warp (32 combos).
 template <bool kMasked, int kMode, bool kCands>
 __device__ __forceinline__ void count_strip(BandSmem& S, const BandArgs& a, const Tile& T, Counter& C,
                                             int slot, int t, int st, int warp, int lane, uint32_t fx,
@@ -408,7 +409,7 @@ __device__ __forceinline__ void count_strip(BandSmem& S, const BandArgs& a, cons
     for (int k = 0; k < kUsed; ++k) {
         const int combo = warp + kWarps * k;
         const int m = combo_band(combo);
-        if (kMode != kModeShared && m >= a.nb) continue;  // warp-uniform
+        if (m >= T.nb || combo_phase(combo) >= T.phases) continue;
         uint32_t n[4];
         // Grouped bands: the slot's own swap plane and phase sense.
         const int gs = kMode == kModeGrouped ? S.gsw[m] : 0;
@@ -469,7 +470,6 @@ __device__ __forceinline__ void band_cta_init(BandSmem& S, int tid) {
 template <int kMode, bool kCands>
 __device__ __forceinline__ bool band_tile(BandSmem& S, const BandArgs& a, int64_t tile, int tid, int lane,
                                           int warp, uint32_t& bar_phase) {
-    const int nb = a.nb;
     const uint32_t thr4 = (uint32_t)min(a.min_size, 128) * 0x01010101u;
     const uint32_t one = a.one;  // 1 at run time: keeps the band add on the multiply pipe
     // Counter constants: the swap sense of the warp's phase and the groups lane 31 may flag
@@ -493,6 +493,15 @@ __device__ __forceinline__ bool band_tile(BandSmem& S, const BandArgs& a, int64_
             (int64_t)T.v0 + (int64_t)a.j0 * a.row_stride >= a.height_v)
             return true;
         T.out_h = min(a.band_h, a.vbase - T.v0);
+        // Bands are ordered by their first row: those with a centre row in this tile are a prefix
+        // (of the copies, with grouped bands).
+        {
+            const int G = kMode == kModeGrouped ? a.groups : 1;
+            const int64_t held = (a.height_v - T.v0 + kPeriod - 1) / kPeriod - a.j0;
+            T.nb = (int)min((int64_t)a.nb, held * G);
+            T.phases = (int64_t)T.u0 + (int64_t)(T.i0 + 1) * kPeriod < a.width_u ? 2 : 1;
+        }
+        const int nb = T.nb;
         const int strips = (T.out_h + 16 + 3) / 4;
         const int batches = (strips + 1) / 2;
         constexpr int kRW = row_words<kMode>();
@@ -740,8 +749,7 @@ __global__ void __launch_bounds__(kTpb, 1) band_scan_kernel(const BandArgs a) {
 // the tile prefix sums and copies that search's arguments into shared memory. Work item i covers
 // tiles args[i].tile_begin .. + (prefix[i+1] - prefix[i]) of its search; prefix[0] need not be 0.
 // One class per launch keeps the kernel as lean as the single-search one (no spills). Stale
-// planes of a previous search with more bands are never read by the grouped-band counter (it skips
-// bands beyond the band count) and are cleared before a shared-LCG tile.
+// planes of a previous tile with more bands are never read: the counter skips bands beyond the tile's.
 template <int kMode, bool kCands>
 __global__ void __launch_bounds__(kTpb, 1) band_batch_kernel(const BandArgs* args, const int64_t* prefix,
                                                              int32_t nsearch, unsigned long long* head) {
@@ -771,18 +779,6 @@ __global__ void __launch_bounds__(kTpb, 1) band_batch_kernel(const BandArgs* arg
         for (int i = tid; i < kArgWords; i += kTpb)
             reinterpret_cast<uint32_t*>(&S.args)[i] = reinterpret_cast<const uint32_t*>(&args[s])[i];
         __syncthreads();
-        if (kMode == kModeShared) {
-            // The shared-LCG counter reads every plane: clear planes of bands this search does
-            // not generate (a previous search may have left bits there).
-            for (int i = tid; i < kRingSlots * kBatchRows * kMaxBands * kWords; i += kTpb) {
-                const int m = (i / kWords) % kMaxBands;
-                if (m >= S.args.nb) {
-                    const int w = i % kWords, r = i / (kWords * kMaxBands);
-                    S.ring[r / kBatchRows][r % kBatchRows][m][w] = 0;
-                }
-            }
-            __syncthreads();
-        }
         if (!band_tile<kMode, kCands>(S, S.args, S.args.tile_begin + t - prefix[s], tid, lane, warp,
                                                      bar_phase)) {
             if (tid == 0) atomicOr(S.args.overflow, 4u);
