@@ -11,9 +11,9 @@
 //      for slime chunks and inserts every slime chunk into a device hash set, so a chunk shared by
 //      neighbouring candidates is evaluated once (high-count sites come in clusters);
 //   2. chunk_kernel -- one thread per (unique chunk, quart): the column's climate noise once
-//      (FP64, 46 octaves in shared memory), then one multi-query tree traversal answers the 17
-//      Deep Dark layers (quart Y -16..0) and the Mushroom Fields layer (quart Y 16) together,
-//      since they differ only in the depth parameter; verdict bits are OR-ed per chunk;
+//      (FP64, 46 octaves in shared memory), then one tree search per biome that only asks whether the
+//      biome's own leaf is the nearest: Mushroom Fields at quart Y 16, and Deep Dark at quart Y -16,
+//      which decides all of its 17 layers (see collect_targets); verdict bits are OR-ed per chunk;
 //   3. verdict_kernel -- one warp per candidate ORs the verdicts of its window's slime chunks.
 #include <algorithm>
 #include <cmath>
@@ -100,7 +100,6 @@ namespace {
 constexpr int kThreads = 128;
 constexpr int kParamSlots = 256;  // node words index parameter ranges with 8 bits
 constexpr uint64_t kEmptyKey = ~0ull;
-constexpr int kDeepLayers = 17;   // quart Y -16..0
 constexpr int32_t kDeepDark = 183, kMushroom = 14;
 
 // Per-device tables: the depth spline and every vendored biome tree (nodes with patches
@@ -112,6 +111,7 @@ struct Tables {
     uint64_t* nodes[BD_TREES] = {};
     int2* params[BD_TREES] = {};
     TreeGeom geom[BD_TREES] = {};
+    Targets deep_dark[BD_TREES] = {}, mushroom[BD_TREES] = {};
 };
 
 Tables& tables() {
@@ -123,6 +123,59 @@ float bits_to_float(int32_t b) {
     float f;
     std::memcpy(&f, &b, 4);
     return f;
+}
+
+// What the verdict search relies on, checked on a tree's words: walks it as the searches do and
+// collects the leaves of the two biomes. True when every box encloses its children's, leaves are met in
+// ascending order at or after the index of each of their ancestors, and the Deep Dark verdict of all
+// layers is decided at the lowest one. That is so when every Deep Dark leaf has the same single depth P
+// and no other leaf's depth range goes past P: with D the depth parameter, which grows downwards, the
+// squared distance to a Deep Dark leaf minus that to any other leaf then falls as D grows (its
+// derivative is at most -2 (P - hi) <= 0 above, inside and below the other's range), so a leaf that
+// is nearer at the deepest layer is nearer at all of them.
+bool collect_targets(const std::vector<uint64_t>& nodes, const std::vector<int2>& param, const TreeGeom& g,
+                     Targets* deep_dark, Targets* mushroom) {
+    bool ok = true;
+    int32_t last = -1, point = 0, deepest_other = INT32_MIN;
+    auto range = [&](int32_t node, int axis) { return param[(nodes[(size_t)node] >> (8 * axis)) & 0xff]; };
+    auto add = [&](Targets* t, int32_t leaf) {
+        if (t->n < kTargetMax) t->leaf[t->n++] = leaf;
+        else ok = false;
+    };
+    struct Frame { int32_t parent, child; int left, d; };
+    std::vector<Frame> stack;
+    stack.push_back({0, (int32_t)((nodes[0] >> 48) & 0xffff), g.order, node_depth(g, 0, 0)});
+    while (!stack.empty()) {
+        Frame& f = stack.back();
+        if (f.left <= 0 || f.child >= g.nnodes) {
+            stack.pop_back();
+            continue;
+        }
+        const int32_t node = f.child, parent = f.parent;
+        const int cd = node_depth(g, node, f.d + 1);
+        f.child += g.steps[f.d];
+        --f.left;
+        for (int a = 0; a < 6 && parent != 0; ++a)  // the root's word is no box: every search enters it
+            ok = ok && range(node, a).x >= range(parent, a).x && range(node, a).y <= range(parent, a).y;
+        ok = ok && node > parent;
+        if (cd < g.depth) {
+            stack.push_back({node, (int32_t)((nodes[(size_t)node] >> 48) & 0xffff), g.order, cd});
+            continue;
+        }
+        ok = ok && node > last;
+        last = node;
+        const int32_t biome = (int32_t)((nodes[(size_t)node] >> 48) & 0xff);
+        const int2 depth = range(node, 4);
+        if (biome == kMushroom) add(mushroom, node);
+        if (biome == kDeepDark) {
+            ok = ok && depth.x == depth.y && (deep_dark->n == 0 || depth.x == point);
+            point = depth.x;
+            add(deep_dark, node);
+        } else {
+            deepest_other = std::max(deepest_other, depth.y);
+        }
+    }
+    return ok && (deep_dark->n == 0 || deepest_other <= point);
 }
 
 }  // namespace
@@ -176,6 +229,11 @@ bool ensure_tables() {
         g.nparams = b.nparams;
         for (int d = 0; d < b.depth; ++d) g.steps[d] = b.steps[d];
         t.geom[k] = g;
+        t.deep_dark[k] = t.mushroom[k] = Targets{};
+        if (!collect_targets(nodes, param, g, &t.deep_dark[k], &t.mushroom[k])) {
+            c.set_error_text("biome tables: tree without the order the verdict search needs");
+            return false;
+        }
         if ((e = cudaMalloc(&t.nodes[k], 8 * nodes.size())) != cudaSuccess ||
             (e = cudaMalloc(&t.params[k], sizeof(int2) * param.size())) != cudaSuccess ||
             (e = cudaMemcpy(t.nodes[k], nodes.data(), 8 * nodes.size(), cudaMemcpyHostToDevice)) != cudaSuccess ||
@@ -307,14 +365,11 @@ __global__ void __launch_bounds__(kThreads) insert_kernel(int64_t seed, const in
 }
 
 // Verdict bits of the quart columns of unique chunks: bit 0 Deep Dark at some quart Y -16..0,
-// bit 1 Mushroom Fields at quart Y 16. NQ queries: 18 (both), 17 (Deep Dark), 1 (Mushroom).
-// Four CTAs per SM (128 registers, no spills): the traversal is latency-bound; twice the warps of
-// the register-limited default (200 registers) ran 23 % more quart columns per second on B200 in a
-// back-to-back comparison on one GPU.
-template <int NQ>
-__global__ void __launch_bounds__(kThreads, 4) chunk_kernel(const Climate* __restrict__ cl, const SplineHead* heads,
+// bit 1 Mushroom Fields at quart Y 16.
+__global__ void __launch_bounds__(kThreads, 6) chunk_kernel(const Climate* __restrict__ cl, const SplineHead* heads,
                                                          const SplinePt* pts, const uint64_t* __restrict__ nodes,
                                                          const int2* __restrict__ param, TreeGeom g,
+                                                         Targets deep_dark, Targets mushroom,
                                                          const int2* __restrict__ chunks, int32_t nchunks,
                                                          unsigned int* chunk_bits, uint32_t want) {
     __shared__ Shared sh;
@@ -328,23 +383,13 @@ __global__ void __launch_bounds__(kThreads, 4) chunk_kernel(const Climate* __res
         const int32_t qx = (int32_t)((uint32_t)ch.x * 4u + (uint32_t)(q >> 2));
         const int32_t qz = (int32_t)((uint32_t)ch.y * 4u + (uint32_t)(q & 3));
         const Column col = column_climate<BD_SPLINE_LEVELS>(sh.cl, sh.heads, sh.pts, qx, qz);
-        const int32_t base[5] = {col.t, col.h, col.c, col.e, col.w};
-        int32_t depth[NQ], biome[NQ];
-        if constexpr (NQ == 1) {
-            depth[0] = depth_at(col.off, 16);
-        } else {
-#pragma unroll
-            for (int i = 0; i < kDeepLayers; ++i) depth[i] = depth_at(col.off, -16 + i);
-            if constexpr (NQ == kDeepLayers + 1) depth[kDeepLayers] = depth_at(col.off, 16);
-        }
-        tree_nearest<NQ>(nodes, sh.param, g, base, depth, biome);
         uint32_t bits = 0;
-        if constexpr (NQ == 1) {
-            bits = biome[0] == kMushroom ? 2u : 0u;
-        } else {
-#pragma unroll
-            for (int i = 0; i < kDeepLayers; ++i) bits |= biome[i] == kDeepDark ? 1u : 0u;
-            if constexpr (NQ == kDeepLayers + 1) bits |= biome[kDeepLayers] == kMushroom ? 2u : 0u;
+        int32_t killer = -1;
+#pragma unroll 1
+        for (uint32_t b = 1; b <= 2; b <<= 1) {
+            if (!(want & b)) continue;
+            const int32_t p[6] = {col.t, col.h, col.c, col.e, depth_at(col.off, b == 1 ? -16 : 16), col.w};
+            if (tree_wins(nodes, sh.param, g, p, b == 1 ? deep_dark : mushroom, killer)) bits |= b;
         }
         if (bits) atomicOr(&chunk_bits[u], bits);
     }
@@ -380,11 +425,8 @@ __global__ void __launch_bounds__(kThreads) query_kernel(const Climate* __restri
     load_shared(sh, cl, heads, pts, param);
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const Column col = column_climate<BD_SPLINE_LEVELS>(sh.cl, sh.heads, sh.pts, xs[i], zs[i]);
-        const int32_t base[5] = {col.t, col.h, col.c, col.e, col.w};
-        const int32_t depth[1] = {depth_at(col.off, ys[i])};
-        int32_t biome[1];
-        tree_nearest<1>(nodes, sh.param, g, base, depth, biome);
-        out[i] = biome[0];
+        const int32_t p[6] = {col.t, col.h, col.c, col.e, depth_at(col.off, ys[i]), col.w};
+        out[i] = tree_biome(nodes, sh.param, g, p);
     }
 }
 
@@ -639,18 +681,9 @@ bool filter_device(BiomeContext* b, const int32_t* dcx, const int32_t* dcz, int3
         }
         const int grid = grid_for((int64_t)nuniq * 16, kThreads);
         const TreeGeom& g = t.geom[b->tree];
-        if (want == 3)
-            chunk_kernel<kDeepLayers + 1><<<grid, kThreads, 0, s>>>(b->d_climate, t.heads, t.pts, t.nodes[b->tree],
-                                                                     t.params[b->tree], g, b->uniq.p, (int32_t)nuniq,
-                                                                     b->chunk_bits.p, want);
-        else if (want == 1)
-            chunk_kernel<kDeepLayers><<<grid, kThreads, 0, s>>>(b->d_climate, t.heads, t.pts, t.nodes[b->tree],
-                                                                 t.params[b->tree], g, b->uniq.p, (int32_t)nuniq,
-                                                                 b->chunk_bits.p, want);
-        else
-            chunk_kernel<1><<<grid, kThreads, 0, s>>>(b->d_climate, t.heads, t.pts, t.nodes[b->tree],
-                                                      t.params[b->tree], g, b->uniq.p, (int32_t)nuniq,
-                                                      b->chunk_bits.p, want);
+        chunk_kernel<<<grid, kThreads, 0, s>>>(b->d_climate, t.heads, t.pts, t.nodes[b->tree], t.params[b->tree], g,
+                                               t.deep_dark[b->tree], t.mushroom[b->tree], b->uniq.p, (int32_t)nuniq,
+                                               b->chunk_bits.p, want);
         ++c.last_launches;
         if ((e = cudaGetLastError()) != cudaSuccess) {
             c.set_error("biome filter: chunks", e);

@@ -93,23 +93,17 @@ enum { kShift = 0, kTemp = 1, kHumid = 2, kCont = 3, kEros = 4, kWeird = 5 };
 __host__ __device__ inline double fade(double t) { return t * t * t * (t * (t * 6.0 - 15.0) + 10.0); }
 __host__ __device__ inline double lerp(double t, double a, double b) { return a + t * (b - a); }
 
-// Gradient dot product of improved noise for hash h: x, y or z (a), with a sign, plus another
-// (b) with a sign: the 12 cube edges, 4 of them repeated.
-__host__ __device__ inline double grad(uint32_t h, double x, double y, double z) {
-    switch (h & 15u) {
-    case 0: case 12: return x + y;
-    case 1: case 14: return -x + y;
-    case 2: return x - y;
-    case 3: return -x - y;
-    case 4: return x + z;
-    case 5: return -x + z;
-    case 6: return x - z;
-    case 7: return -x - z;
-    case 8: return y + z;
-    case 9: case 13: return -y + z;
-    case 10: return y - z;
-    default: return -y - z;  // 11, 15
-    }
+// Gradient dot product of improved noise for hash h: the 12 cube edges, 4 of them repeated, as u + v
+// with u, v two of x, y, z and a sign each (u = x below 8, else y; v = y below 4, x at 12 and 14, else
+// z; bit 0 negates u and bit 1 v). Selects and sign flips instead of a 12-way branch, which a warp ran
+// nearly all of.
+__device__ __forceinline__ double with_sign(double v, uint32_t flip) {
+    return __hiloint2double(__double2hiint(v) ^ (int)flip, __double2loint(v));
+}
+__device__ __forceinline__ double grad(uint32_t h, double x, double y, double z) {
+    const double u = h & 8u ? y : x;
+    const double v = (h & 13u) == 12u ? x : h & 12u ? z : y;
+    return with_sign(u, h << 31) + with_sign(v, (h << 30) & 0x80000000u);
 }
 
 // Octave set initialisation on the host (the permutation shuffle is serial): two seeds from the
@@ -155,21 +149,28 @@ __device__ __forceinline__ double perlin_sample(const Octave& p, double x, doubl
     return lerp(tz, l1, l5);
 }
 
-__device__ __forceinline__ double octaves_sample(const Octave* o, int n, double x, double y, double z) {
-    double v = 0.0;
-    for (int i = 0; i < n; ++i) {
-        const double f = o[i].lac;
-        const double s = perlin_sample(o[i], x * f, y * f, z * f);
-        v += o[i].amp * s;
-    }
-    return v;
-}
-
+// The two octave sets of a noise, the second at 337/331 of the position. One loop body for both: the
+// seven samples of a quart column would otherwise inline it fourteen times.
 __device__ __forceinline__ double noise_sample(const Climate& c, int s, double x, double y, double z) {
     const Noise& n = c.noise[s];
     const double f = 337.0 / 331.0;
-    double v = octaves_sample(c.oct + n.first, n.na, x, y, z);
-    v += octaves_sample(c.oct + n.first + n.na, n.nb, x * f, y * f, z * f);
+    double v = 0.0;
+#pragma unroll 1
+    for (int set = 0; set < 2; ++set) {
+        const Octave* o = c.oct + n.first + (set ? n.na : 0);
+        const int count = set ? n.nb : n.na;
+        double acc = 0.0;
+#pragma unroll 1
+        for (int i = 0; i < count; ++i) {
+            const double l = o[i].lac;
+            const double p = perlin_sample(o[i], x * l, y * l, z * l);
+            acc += o[i].amp * p;
+        }
+        v = set ? v + acc : acc;
+        x *= f;
+        y *= f;
+        z *= f;
+    }
     return v * n.amp;
 }
 
@@ -239,16 +240,24 @@ template <int SPLINE_LEVELS>
 __device__ __forceinline__ Column column_climate(const Climate& cl, const SplineHead* heads, const SplinePt* pts,
                                                  int32_t xi, int32_t zi) {
     const double x = (double)xi, z = (double)zi;
-    const double px = x + noise_sample(cl, kShift, x, 0.0, z) * 4.0;
-    const double pz = z + noise_sample(cl, kShift, z, x, 0.0) * 4.0;
-    const float c = (float)noise_sample(cl, kCont, px, 0.0, pz);
-    const float e = (float)noise_sample(cl, kEros, px, 0.0, pz);
-    const float w = (float)noise_sample(cl, kWeird, px, 0.0, pz);
+    double at[2];  // shifted position
+#pragma unroll 1
+    for (int k = 0; k < 2; ++k) {
+        const double d = noise_sample(cl, kShift, k ? z : x, k ? x : 0.0, k ? 0.0 : z) * 4.0;
+        at[0] = k ? at[0] : x + d;
+        at[1] = z + d;
+    }
+    float v[6];  // by noise, kTemp .. kWeird
+#pragma unroll 1
+    for (int s = kTemp; s <= kWeird; ++s) {
+        const float d = (float)noise_sample(cl, s, at[0], 0.0, at[1]);
+#pragma unroll
+        for (int k = kTemp; k <= kWeird; ++k) v[k] = s == k ? d : v[k];
+    }
+    const float c = v[kCont], e = v[kEros], w = v[kWeird], t = v[kTemp], h = v[kHumid];
     const float in[4] = {c, e, peaks_valleys(w), w};
     Column col;
     col.off = spline_eval<SPLINE_LEVELS>(heads, pts, 0, in) + 0.015f;
-    const float t = (float)noise_sample(cl, kTemp, px, 0.0, pz);
-    const float h = (float)noise_sample(cl, kHumid, px, 0.0, pz);
     col.t = (int32_t)(10000.0f * t);
     col.h = (int32_t)(10000.0f * h);
     col.c = (int32_t)(10000.0f * c);
@@ -272,11 +281,6 @@ struct TreeGeom {
     int32_t steps[8];
 };
 
-__device__ __forceinline__ int64_t axis_d2(int32_t v, int2 r) {
-    const int64_t d = v > r.y ? (int64_t)v - r.y : v < r.x ? (int64_t)r.x - v : 0;
-    return d * d;
-}
-
 // Distance of v to the range r along one axis. kWide: exact for every int32 v (64-bit
 // differences); otherwise 32-bit differences, exact while |v| <= 2^30 (range bounds are within
 // +-12,000, so no difference overflows).
@@ -293,37 +297,35 @@ __device__ __forceinline__ uint32_t axis_gap(int32_t v, int2 r) {
 // as the reference's int64 / uint64 arithmetic gives for these magnitudes).
 __device__ __forceinline__ uint64_t add_sq(uint64_t acc, uint32_t g) { return acc + (uint64_t)g * g; }
 
-// Nearest leaves of NQ queries that differ only in the depth axis (axis 4), in one traversal.
-// Each query follows exactly the reference's branch and bound (MinecraftGPUNoise.cu:686-809):
-// children of a node at tree depth d are `order` nodes steps[d] apart (a node whose subtree would
-// run past the end descends in place), a child is entered when its box is strictly closer than
-// the query's best leaf, and a leaf replaces the best only when strictly closer. Per stack level
-// a bit mask keeps the queries that entered the subtree; the other queries neither descend nor
-// update there, so every query visits and decides exactly as a search of its own would.
-// Returns the biome ids (link byte of the best leaf) in biome[].
-template <int NQ, bool kWide>
-__device__ __forceinline__ void tree_nearest_impl(const uint64_t* __restrict__ nodes, const int2* __restrict__ param,
-                                                  const TreeGeom& g, const int32_t base[5],
-                                                  const int32_t (&depth)[NQ], int32_t (&biome)[NQ]) {
-    constexpr int kMaxDepth = 8;
-    static_assert(NQ <= 32, "query mask is 32 bits");
-    uint64_t ds[NQ];
-    int32_t best[NQ];
+// A node word: parameter indices of the six axes in bytes 0..5 (depth in byte 4), then the first
+// child's node index, or a leaf's biome id. `order` children lie steps[d] apart below a node at tree
+// depth d; a node whose subtree would run past the end descends in place.
+template <bool kWide>
+__device__ __forceinline__ uint64_t node_d2(uint64_t node, const int2* __restrict__ param, const int32_t (&p)[6]) {
+    uint64_t d = 0;
 #pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-        ds[q] = ~0ull;
-        best[q] = 0;
-    }
-    // Stack level: next child (bits 0-15), children left (16-23), tree depth (24-31); query mask.
-    uint32_t st_node[kMaxDepth], st_mask[kMaxDepth];
+    for (int a = 0; a < 6; ++a) d = add_sq(d, axis_gap<kWide>(p[a], param[(node >> (8 * a)) & 0xff]));
+    return d;
+}
+__host__ __device__ __forceinline__ int node_depth(const TreeGeom& g, int32_t node, int d) {
+    while (d < g.depth && node + g.steps[d] >= g.nnodes) ++d;
+    return d;
+}
+
+// Index of the nearest leaf of parameters p (temperature, humidity, continentalness, erosion, depth,
+// weirdness): the reference's branch and bound (MinecraftGPUNoise.cu:686-809). A child is entered
+// when its box is strictly closer than the best leaf, and a leaf replaces the best only when strictly
+// closer, so with boxes that enclose their leaves the answer is the first of the nearest leaves.
+template <bool kWide>
+__device__ __forceinline__ int32_t tree_nearest_impl(const uint64_t* __restrict__ nodes, const int2* __restrict__ param,
+                                                     const TreeGeom& g, const int32_t (&p)[6]) {
+    constexpr int kMaxDepth = 8;
+    uint64_t ds = ~0ull;
+    int32_t best = 0;
+    // Stack level: next child (bits 0-15), children left (16-23), tree depth (24-31).
+    uint32_t st_node[kMaxDepth];
     int sp = 0;
-    // Root: node 0 at depth 0, every query active.
-    {
-        int d = 0;
-        while (d < g.depth && 0 + g.steps[d] >= g.nnodes) ++d;
-        st_node[0] = (uint32_t)((nodes[0] >> 48) & 0xffff) | ((uint32_t)g.order << 16) | ((uint32_t)d << 24);
-        st_mask[0] = NQ == 32 ? 0xffffffffu : ((1u << NQ) - 1u);
-    }
+    st_node[0] = (uint32_t)((nodes[0] >> 48) & 0xffff) | ((uint32_t)g.order << 16) | ((uint32_t)node_depth(g, 0, 0) << 24);
     while (sp >= 0) {
         const uint32_t top = st_node[sp];
         const int32_t child = (int32_t)(top & 0xffff);
@@ -333,57 +335,125 @@ __device__ __forceinline__ void tree_nearest_impl(const uint64_t* __restrict__ n
             continue;
         }
         st_node[sp] = (uint32_t)(child + g.steps[d]) | ((uint32_t)(left - 1) << 16) | ((uint32_t)d << 24);
-        const uint32_t active = st_mask[sp];
         const uint64_t node = nodes[child];
-        // The five depth-independent axes once, then the depth axis per query.
-        uint64_t b5 = add_sq(0, axis_gap<kWide>(base[0], param[node & 0xff]));
-        b5 = add_sq(b5, axis_gap<kWide>(base[1], param[(node >> 8) & 0xff]));
-        b5 = add_sq(b5, axis_gap<kWide>(base[2], param[(node >> 16) & 0xff]));
-        b5 = add_sq(b5, axis_gap<kWide>(base[3], param[(node >> 24) & 0xff]));
-        b5 = add_sq(b5, axis_gap<kWide>(base[4], param[(node >> 40) & 0xff]));
-        const int2 rd = param[(node >> 32) & 0xff];
-        uint32_t enter = 0;
-#pragma unroll
-        for (int q = 0; q < NQ; ++q)
-            if (((active >> q) & 1u) && add_sq(b5, axis_gap<kWide>(depth[q], rd)) < ds[q]) enter |= 1u << q;
-        if (!enter) continue;
-        // The child sits at depth d + 1; a subtree that would run past the end descends in place.
-        int cd = d + 1;
-        while (cd < g.depth && child + g.steps[cd] >= g.nnodes) ++cd;
+        const uint64_t dist = node_d2<kWide>(node, param, p);
+        if (dist >= ds) continue;
+        const int cd = node_depth(g, child, d + 1);
         if (cd >= g.depth) {
-            // A leaf: each entering query takes it (its distance is below the query's best).
-#pragma unroll
-            for (int q = 0; q < NQ; ++q)
-                if ((enter >> q) & 1u) {
-                    ds[q] = add_sq(b5, axis_gap<kWide>(depth[q], rd));
-                    best[q] = child;
-                }
+            ds = dist;
+            best = child;
             continue;
         }
-        ++sp;
-        st_node[sp] = (uint32_t)((node >> 48) & 0xffff) | ((uint32_t)g.order << 16) | ((uint32_t)cd << 24);
-        st_mask[sp] = enter;
+        st_node[++sp] = (uint32_t)((node >> 48) & 0xffff) | ((uint32_t)g.order << 16) | ((uint32_t)cd << 24);
     }
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) biome[q] = (int32_t)((nodes[best[q]] >> 48) & 0xff);
+    return best;
 }
 
 // The 32-bit-gap traversal when every coordinate is within +-2^30 (always, for climate values and
 // the depths of quart Y within the world), else the 64-bit one; both give the same leaves.
-template <int NQ>
-__device__ __forceinline__ void tree_nearest(const uint64_t* __restrict__ nodes, const int2* __restrict__ param,
-                                             const TreeGeom& g, const int32_t base[5], const int32_t (&depth)[NQ],
-                                             int32_t (&biome)[NQ]) {
+__device__ __forceinline__ bool wide_params(const int32_t (&p)[6]) {
     constexpr int32_t kLim = 1 << 30;
     bool wide = false;
 #pragma unroll
-    for (int i = 0; i < 5; ++i) wide |= base[i] > kLim || base[i] < -kLim;
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) wide |= depth[q] > kLim || depth[q] < -kLim;
-    if (wide)
-        tree_nearest_impl<NQ, true>(nodes, param, g, base, depth, biome);
-    else
-        tree_nearest_impl<NQ, false>(nodes, param, g, base, depth, biome);
+    for (int i = 0; i < 6; ++i) wide |= p[i] > kLim || p[i] < -kLim;
+    return wide;
+}
+__device__ __forceinline__ int32_t tree_biome(const uint64_t* __restrict__ nodes, const int2* __restrict__ param,
+                                              const TreeGeom& g, const int32_t (&p)[6]) {
+    const int32_t leaf = wide_params(p) ? tree_nearest_impl<true>(nodes, param, g, p)
+                                        : tree_nearest_impl<false>(nodes, param, g, p);
+    return (int32_t)((nodes[leaf] >> 48) & 0xff);
+}
+
+// Leaves of one biome (at most kTargetMax of them), for a verdict "is the nearest leaf one of these".
+constexpr int kTargetMax = 4;
+struct Targets {
+    int32_t n;
+    int32_t leaf[kTargetMax];
+};
+
+// Whether the nearest leaf of parameters p is a leaf of `t`. The nearest of t's own leaves sets a
+// bound, and the search only asks whether any other leaf is nearer (or as near and earlier in leaf
+// order, which is the order the reference visits them in): it ends at the first one. At each node all
+// children are measured and the nearest is followed first, so that a column far from the biome's
+// climate ends after one descent (about 30 node distances; the full search for the nearest leaf of
+// 18 depths took 168,000 instructions a warp, noise included). `killer`: a leaf to try first, and the
+// leaf that ended the search.
+template <bool kWide>
+__device__ __forceinline__ bool tree_wins_impl(const uint64_t* __restrict__ nodes, const int2* __restrict__ param,
+                                               const TreeGeom& g, const int32_t (&p)[6], const Targets& t, int32_t& killer) {
+    constexpr int kMaxDepth = 8;
+    uint64_t bound = ~0ull;
+    int32_t first = 0;  // the target leaf at `bound`
+    for (int i = 0; i < t.n; ++i) {  // ascending leaves: the first of the nearest
+        const uint64_t dist = node_d2<kWide>(nodes[t.leaf[i]], param, p);
+        if (dist < bound) {
+            bound = dist;
+            first = t.leaf[i];
+        }
+    }
+    // Nearer than the bound, or as near and earlier (a subtree's leaves come after its own index).
+    auto beats = [&](uint64_t dist, int32_t node) { return dist < bound || (dist == bound && node < first); };
+    if (killer >= 0 && beats(node_d2<kWide>(nodes[killer], param, p), killer)) return false;
+    // Stack level: first child (bits 0-15), tree depth (16-23); the children still to enter.
+    uint32_t st_node[kMaxDepth], st_todo[kMaxDepth];
+    int sp = -1;
+    int32_t inner = (int32_t)((nodes[0] >> 48) & 0xffff);
+    int d = node_depth(g, 0, 0);
+    bool measure = true;
+    uint32_t todo = 0;
+    int pick = 0;
+    for (;;) {
+        if (measure) {  // children that can hold a leaf that beats the bound, and the nearest of them
+            todo = 0;
+            uint64_t nearest = ~0ull;
+#pragma unroll 2
+            for (int k = 0; k < g.order; ++k) {
+                const int32_t child = inner + k * g.steps[d];
+                if (child >= g.nnodes) break;
+                const uint64_t dist = node_d2<kWide>(nodes[child], param, p);
+                if (!beats(dist, child)) continue;
+                todo |= 1u << k;
+                if (dist < nearest) {
+                    nearest = dist;
+                    pick = k;
+                }
+            }
+            measure = false;
+        }
+        if (!todo) {
+            if (sp < 0) return true;
+            inner = (int32_t)(st_node[sp] & 0xffff);
+            d = (int)(st_node[sp] >> 16);
+            todo = st_todo[sp--];
+            pick = __ffs(todo) - 1;
+        }
+        const int32_t child = inner + pick * g.steps[d];
+        todo &= ~(1u << pick);
+        const int cd = node_depth(g, child, d + 1);
+        if (cd >= g.depth) {
+            bool own = false;
+            for (int i = 0; i < t.n; ++i) own |= t.leaf[i] == child;
+            if (!own) {
+                killer = child;
+                return false;
+            }
+            pick = __ffs(todo) - 1;
+            continue;
+        }
+        if (todo) {
+            st_node[++sp] = (uint32_t)inner | ((uint32_t)d << 16);
+            st_todo[sp] = todo;
+        }
+        inner = (int32_t)((nodes[child] >> 48) & 0xffff);
+        d = cd;
+        measure = true;
+    }
+}
+__device__ __forceinline__ bool tree_wins(const uint64_t* __restrict__ nodes, const int2* __restrict__ param,
+                                          const TreeGeom& g, const int32_t (&p)[6], const Targets& t, int32_t& killer) {
+    return wide_params(p) ? tree_wins_impl<true>(nodes, param, g, p, t, killer)
+                          : tree_wins_impl<false>(nodes, param, g, p, t, killer);
 }
 
 }  // namespace biome
