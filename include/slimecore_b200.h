@@ -185,7 +185,7 @@ int32_t slime_b200_microbench(int32_t kind, int32_t iters, double* lane_ops_per_
  * loads the library holds until the process exits; the call makes no cudaMalloc, cudaFree,
  * cudaMallocHost or host heap allocation (error texts go to a fixed buffer). Limits: rd_max <= 8191
  * and max_results <= 65536; larger requests return -1 with an error text (slime_b200_last_error).
- * A call can also return -1 if a single 64-row band of the area holds more than about 327k centres
+ * A call can also return -1 if a single 64-row band of the area holds more than about 349k centres
  * at or above the count gate its max_results implies (possible only with max_results near 65536
  * and a wide area). The first call on a device looks up the array's device address (set-up) and
  * caches it per device ordinal, so make that first call before any stream capture; a device

@@ -49,6 +49,7 @@ bool Context::ensure_device() {
         return false;
     }
     cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device);
+    general_grid = general_max_grid();
     if (cudaEventCreate(&ev_a) != cudaSuccess || cudaEventCreate(&ev_b) != cudaSuccess) {
         set_error("events", cudaErrorUnknown);
         return false;
@@ -67,7 +68,6 @@ void Context::release_extra() {}
 void Context::release() {
     release_biome();
     xt.free();
-    zt.free();
     hits.free();
     counters.free();
     hist.free();
@@ -147,18 +147,6 @@ bool Context::ensure_y_tables() {
 
 namespace {
 
-// log P(Binomial(221, 0.1) >= s): the expected share of centres whose count reaches s.
-double log_tail(int s) {
-    if (s <= 0) return 0.0;
-    double acc = -INFINITY;
-    for (int k = s; k <= 221; ++k) {
-        const double lp = std::lgamma(222.0) - std::lgamma(k + 1.0) - std::lgamma(222.0 - k) +
-                          k * std::log(0.1) + (221 - k) * std::log(0.9);
-        acc = std::max(acc, lp) + std::log1p(std::exp(-std::fabs(acc - lp)));
-    }
-    return acc;
-}
-
 inline bool hit_better(const Hit& a, const Hit& b) { return hit_order(a, b); }
 
 void keep_best(std::vector<Hit>& v, size_t k) {
@@ -188,52 +176,40 @@ bool Context::scan_general(const SearchSpec& q, std::vector<Hit>& best, std::vec
     const int64_t width = 2 * q.rd_max + 1;
     const int32_t area_x0 = (int32_t)((int64_t)q.center_x - q.rd_max);
     const int32_t area_z0 = (int32_t)((int64_t)q.center_z - q.rd_max);
-    const size_t nterms = (size_t)width + 16;
     cudaError_t e;
-    if ((e = xt.reserve(nterms)) != cudaSuccess || (e = zt.reserve(nterms)) != cudaSuccess ||
-        (e = counters.reserve(4)) != cudaSuccess || (e = hist.reserve(kHistBins)) != cudaSuccess ||
-        (e = hits.reserve(hit_capacity(q.max_results))) != cudaSuccess) {
+    if ((e = hits.reserve(kScanHeader + hit_capacity(q.max_results))) != cudaSuccess) {
         set_error("alloc", e);
         return false;
     }
-    if ((e = launch_terms(xt.ptr, area_x0 - 8, (int32_t)nterms, zt.ptr, area_z0 - 8, (int32_t)nterms,
-                          q.seed, stream)) != cudaSuccess) {
-        set_error("terms", e);
-        return false;
-    }
-    ++last_launches;
-    const bool narrow = width < 8192;
-    const int out_w = general_out_width(narrow);
+    const int out_w = general_out_width();
     const int tiles_x = (int)((width + out_w - 1) / out_w);
-    const int max_grid = general_max_grid(narrow);
     const int64_t height = width;
-    // Enough tiles for ~2 waves of the persistent grid, but bands of at least 64 rows.
-    int band_h = (int)std::min<int64_t>(2048, std::max<int64_t>(64, (height * tiles_x) / (2LL * max_grid) + 1));
-    const uint64_t cap = hits.count;
+    const int band_h = general_band_rows(width, height, sm_count);
+    const uint64_t cap = hits.count - kScanHeader;
+    Hit* const first_hits = reinterpret_cast<Hit*>((char*)pinned + kScanHeaderBytes);
     const double area = (double)width * (double)height;
 
     // Materialise only counts that keep the expected emission well inside the buffer; the exact
     // histogram decides afterwards whether a lower gate is needed (second pass).
     int emit_min = q.min_size;
-    while (emit_min < q.max_size && area * std::exp(log_tail(emit_min)) > (double)cap / 8.0 &&
-           area * std::exp(log_tail(emit_min + 1)) >= 4.0 * q.max_results)
+    while (emit_min < q.max_size && area * tail_share(emit_min) > (double)cap / 8.0 &&
+           area * tail_share(emit_min + 1) >= 4.0 * q.max_results)
         ++emit_min;
 
     for (int pass = 0; pass < 3; ++pass) {
         best.clear();
         std::fill(h.begin(), h.end(), 0u);
         // Rows per launch: ~4e10 centres, and an expected emission of at most cap / 4.
-        const double per_row = (double)width * std::exp(log_tail(emit_min));
+        const double per_row = (double)width * tail_share(emit_min);
         int64_t slab = std::min<int64_t>(height, std::max<int64_t>(band_h, (int64_t)(4e10 / width)));
         if (per_row > 0) slab = std::min<int64_t>(slab, std::max<int64_t>(band_h, (int64_t)(cap / 4 / per_row)));
-        slab = std::max<int64_t>(band_h, (slab / band_h) * band_h);
+        slab = (slab + band_h - 1) / band_h * band_h;  // whole patches: an area that fits runs in one launch
         for (int64_t z0 = 0; z0 < height;) {
             while (paused.load() && !cancel.load()) std::this_thread::sleep_for(std::chrono::milliseconds(20));
             if (cancel.load()) { cancelled = true; return true; }
             const int32_t rows = (int32_t)std::min<int64_t>(slab, height - z0);
             ScanArgs a{};
-            a.xt = xt.ptr;
-            a.zt = zt.ptr;
+            a.seed = q.seed;
             a.area_x0 = area_x0;
             a.area_z0 = area_z0;
             a.width = (int32_t)width;
@@ -249,21 +225,20 @@ bool Context::scan_general(const SearchSpec& q, std::vector<Hit>& best, std::vec
             a.rd_min_sq = q.rd_min * q.rd_min;
             a.center_x = q.center_x;
             a.center_z = q.center_z;
-            a.out = hits.ptr;
+            a.out = hits.ptr + kScanHeader;
             a.cap = cap;
-            a.emitted = counters.ptr;
-            a.hist = hist.ptr;
+            a.emitted = reinterpret_cast<unsigned long long*>(hits.ptr);
+            a.hist = reinterpret_cast<unsigned int*>((char*)hits.ptr + 64);
             const int64_t tiles = (int64_t)a.tiles_x * a.tiles_z;
             const auto t0 = std::chrono::steady_clock::now();
             // Per-slab counter and histogram: a slab that overflows the buffer is redone in halves
             // and its partial counts must not be kept.
-            if ((e = cudaMemsetAsync(counters.ptr, 0, 8, stream)) != cudaSuccess ||
-                (e = cudaMemsetAsync(hist.ptr, 0, kHistBins * 4, stream)) != cudaSuccess ||
+            if ((e = cudaMemsetAsync(hits.ptr, 0, kScanHeaderBytes, stream)) != cudaSuccess ||
                 (e = cudaEventRecord(ev_a, stream)) != cudaSuccess ||
-                (e = launch_general_scan(a, narrow, (int)std::min<int64_t>(tiles, max_grid), stream)) != cudaSuccess ||
+                (e = launch_general_scan(a, (int)std::min<int64_t>(tiles, general_grid), stream)) != cudaSuccess ||
                 (e = cudaEventRecord(ev_b, stream)) != cudaSuccess ||
-                (e = cudaMemcpyAsync(pinned, counters.ptr, 8, cudaMemcpyDeviceToHost, stream)) != cudaSuccess ||
-                (e = cudaMemcpyAsync((char*)pinned + 64, hist.ptr, kHistBins * 4, cudaMemcpyDeviceToHost, stream)) != cudaSuccess ||
+                (e = cudaMemcpyAsync(pinned, hits.ptr, kScanHeaderBytes + kScanFirstHits * sizeof(Hit), cudaMemcpyDeviceToHost,
+                                     stream)) != cudaSuccess ||
                 (e = cudaStreamSynchronize(stream)) != cudaSuccess) {
                 set_error("scan", e);
                 return false;
@@ -286,9 +261,12 @@ bool Context::scan_general(const SearchSpec& q, std::vector<Hit>& best, std::vec
             if (emitted) {
                 const size_t old = best.size();
                 best.resize(old + emitted);
-                if ((e = cudaMemcpyAsync(best.data() + old, hits.ptr, emitted * sizeof(Hit),
-                                         cudaMemcpyDeviceToHost, stream)) != cudaSuccess ||
-                    (e = cudaStreamSynchronize(stream)) != cudaSuccess) {
+                const size_t n0 = std::min<size_t>(emitted, kScanFirstHits);
+                std::copy(first_hits, first_hits + n0, best.begin() + (ptrdiff_t)old);
+                if (emitted > n0 &&
+                    ((e = cudaMemcpyAsync(best.data() + old + n0, hits.ptr + kScanHeader + n0, (emitted - n0) * sizeof(Hit),
+                                          cudaMemcpyDeviceToHost, stream)) != cudaSuccess ||
+                     (e = cudaStreamSynchronize(stream)) != cudaSuccess)) {
                     set_error("copy", e);
                     return false;
                 }

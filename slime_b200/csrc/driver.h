@@ -88,6 +88,14 @@ inline size_t hit_capacity(int32_t max_results) {
     return k > (4u << 20) ? k : (4u << 20);
 }
 
+// The general scan keeps its counter, histogram and hits in one buffer, so that one copy brings back a
+// small search: the first kScanHeader hit records hold the counter (byte 0) and the histogram (byte 64).
+constexpr size_t kScanHeader = 128;
+constexpr size_t kScanHeaderBytes = kScanHeader * sizeof(Hit);
+constexpr size_t kScanFirstHits = 2048;  // hits copied with the header
+static_assert(64 + kHistBins * 4 <= kScanHeaderBytes && kScanHeaderBytes + kScanFirstHits * sizeof(Hit) <= kPinnedBytes,
+              "scan header");
+
 // Chunk coordinates to the reference's 32-bit block coordinate (wraps like the reference).
 inline int32_t block_of(int32_t c) { return (int32_t)((uint32_t)c * 16u + 8u); }
 
@@ -111,7 +119,7 @@ struct Context {
     // Last error text: a fixed buffer, so that recording an error never allocates.
     char last_error[256] = {};
 
-    DeviceBuffer<uint64_t> xt, zt;
+    DeviceBuffer<uint64_t> xt;
     DeviceBuffer<Hit> hits;
     DeviceBuffer<unsigned long long> counters;
     DeviceBuffer<unsigned int> hist;
@@ -184,6 +192,7 @@ struct Context {
     double last_kernel_ms = 0.0;
     int64_t last_launches = 0;
     cudaEvent_t ev_a = nullptr, ev_b = nullptr;
+    int general_grid = 0;  // resident CTAs of the general scan on this device
 
     void set_error(const char* where, cudaError_t e);
     void set_error_text(const char* text);

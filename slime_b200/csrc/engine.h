@@ -14,12 +14,11 @@ constexpr int kHistBins = 222;  // window counts 0..221
 
 // One launch of the general scan over rows [slab_z0, slab_z0 + slab_h) of a search area.
 struct ScanArgs {
-    const uint64_t* xt;    // xt[i] = x_term(area_x0 - 8 + i), i < width + 16
-    const uint64_t* zt;    // zt[j] = z_term(area_z0 - 8 + j) + seed, j < height + 16
+    int64_t seed;
     int32_t area_x0, area_z0;  // chunk coordinates of the first centre of the area
     int32_t width, height;     // centres per axis
     int32_t slab_z0, slab_h;   // centre rows of this launch
-    int32_t band_h;            // centre rows per tile
+    int32_t band_h;            // centre rows per patch (a multiple of 8, at most 128)
     int32_t tiles_x, tiles_z;
     int32_t min_size, max_size, emit_min;
     int64_t rd_min_sq;
@@ -30,14 +29,11 @@ struct ScanArgs {
     unsigned int* hist;           // kHistBins counters of every kept centre by count
 };
 
-// Tile geometry of the general scan: `narrow` = 256-chunk input tiles, else 1024.
-int general_out_width(bool narrow);
-cudaError_t launch_general_scan(const ScanArgs& a, bool narrow, int grid, cudaStream_t s);
-int general_max_grid(bool narrow);
-
-// Fills xt/zt for an area (x terms, and z terms with the seed folded in).
-cudaError_t launch_terms(uint64_t* xt, int32_t x0, int32_t nx, uint64_t* zt, int32_t z0,
-                         int32_t nz, int64_t seed, cudaStream_t s);
+// Patch geometry of the general scan.
+int general_out_width();
+int general_band_rows(int64_t width, int64_t height, int sm_count);
+int general_max_grid();
+cudaError_t launch_general_scan(const ScanArgs& a, int grid, cudaStream_t s);
 
 // Precise AFK scoring (SlimeCore.cpp:654-726 semantics).
 struct PreciseArgs {

@@ -29,9 +29,8 @@ namespace {
 
 constexpr int64_t kMaxRadius = 8191;                         // width <= 16,383 centres
 constexpr int32_t kMaxResults = 65536;
-constexpr size_t kTermBytes = (2 * kMaxRadius + 1 + 16) * sizeof(uint64_t);
 constexpr size_t kScratchBytes = 4u << 20;                   // 4 MiB per device
-constexpr size_t kHitsOffset = 2 * kTermBytes + 1024;        // after xt, zt, counters, histogram
+constexpr size_t kHitsOffset = 1024;                         // after counter and histogram
 constexpr uint64_t kHitCap = (kScratchBytes - kHitsOffset) / sizeof(Hit);
 constexpr int kMaxDevices = 64;
 constexpr int kCopyChunk = 2048;                             // hits copied back per memcpy
@@ -93,28 +92,22 @@ int64_t search_noalloc(int64_t seed, int64_t rd_max, int32_t min_size, int32_t m
     unsigned char* base = nullptr;
     if (!scratch_for_current_device(&base)) return -1;
     const int64_t width = 2 * rd_max + 1, height = width;
-    uint64_t* xt = reinterpret_cast<uint64_t*>(base);
-    uint64_t* zt = reinterpret_cast<uint64_t*>(base + kTermBytes);
-    unsigned long long* emitted = reinterpret_cast<unsigned long long*>(base + 2 * kTermBytes);
-    unsigned int* hist = reinterpret_cast<unsigned int*>(base + 2 * kTermBytes + 64);
+    unsigned long long* emitted = reinterpret_cast<unsigned long long*>(base);
+    unsigned int* hist = reinterpret_cast<unsigned int*>(base + 64);
     Hit* hits = reinterpret_cast<Hit*>(base + kHitsOffset);
     const int32_t x0 = (int32_t)((int64_t)cx - rd_max), z0 = (int32_t)((int64_t)cz - rd_max);
     cudaStream_t s = 0;  // the legacy default stream: creating a stream is avoided too
-    cudaError_t e = launch_terms(xt, x0 - 8, (int32_t)(width + 16), zt, z0 - 8, (int32_t)(width + 16), seed, s);
-    if (e != cudaSuccess) { ctx().set_error("no-alloc search: terms", e); return -1; }
-
-    const bool narrow = width < 8192;
-    const int out_w = general_out_width(narrow);
+    cudaError_t e;
+    const int out_w = general_out_width();
     const int tiles_x = (int)((width + out_w - 1) / out_w);
-    const int max_grid = general_max_grid(narrow);
+    const int max_grid = general_max_grid();
     const int band_h = 64;
     const int32_t tiles_z_all = (int32_t)((height + band_h - 1) / band_h);
 
     auto run = [&](int32_t emit_min, int32_t slab_z0, int32_t slab_h, uint64_t* n_emitted,
                    uint32_t* hist_out) -> bool {
         ScanArgs a{};
-        a.xt = xt;
-        a.zt = zt;
+        a.seed = seed;
         a.area_x0 = x0;
         a.area_z0 = z0;
         a.width = (int32_t)width;
@@ -139,7 +132,7 @@ int64_t search_noalloc(int64_t seed, int64_t rd_max, int32_t min_size, int32_t m
         // Counter and histogram keep the previous call's contents: clear them first.
         if ((e = cudaMemsetAsync(emitted, 0, 8, s)) != cudaSuccess ||
             (e = cudaMemsetAsync(hist, 0, kHistBins * 4, s)) != cudaSuccess ||
-            (e = launch_general_scan(a, narrow, (int)std::min<int64_t>(tiles, max_grid), s)) != cudaSuccess ||
+            (e = launch_general_scan(a, (int)std::min<int64_t>(tiles, max_grid), s)) != cudaSuccess ||
             (e = cudaMemcpyAsync(&n, emitted, 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
             (hist_out && (e = cudaMemcpyAsync(hist_out, hist, kHistBins * 4, cudaMemcpyDeviceToHost, s)) != cudaSuccess) ||
             (e = cudaStreamSynchronize(s)) != cudaSuccess) {
