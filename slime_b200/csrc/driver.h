@@ -92,7 +92,7 @@ inline size_t hit_capacity(int32_t max_results) {
 // small search: the first kScanHeader hit records hold the counter (byte 0) and the histogram (byte 64).
 constexpr size_t kScanHeader = 128;
 constexpr size_t kScanHeaderBytes = kScanHeader * sizeof(Hit);
-constexpr size_t kScanFirstHits = 2048;  // hits copied with the header
+constexpr size_t kScanFirstHits = 4096;  // hits copied with the header
 static_assert(64 + kHistBins * 4 <= kScanHeaderBytes && kScanHeaderBytes + kScanFirstHits * sizeof(Hit) <= kPinnedBytes,
               "scan header");
 
@@ -214,7 +214,8 @@ struct Context {
     // fewer than max_results pass and `best` misses sites of the area, kNeedMoreSites.
     int64_t finish(const SearchSpec& q, std::vector<Hit>& best, const std::vector<uint32_t>& h,
                    ExtChunkResult* results);
-    int64_t finish_biome(const SearchSpec& q, std::vector<Hit>& best, int64_t total, ExtChunkResult* results);
+    int64_t finish_biome(const SearchSpec& q, std::vector<Hit>& best, const std::vector<uint32_t>& h, int64_t total,
+                         ExtChunkResult* results);
     // Sites examined and excluded by the biome filter in the last search.
     int64_t last_biome_examined = 0, last_biome_excluded = 0;
     // Many searches: those the independent-band kernel can take share one persistent launch.
