@@ -34,22 +34,32 @@ constexpr uint32_t kInv5 = 0xCCCCCCCDu;
 constexpr uint32_t kTwoInv5 = 2u * kInv5;                         // mod 2^32
 constexpr uint32_t kMulH = (uint32_t)((2ULL * 0x5DEECE66DULL * kInv5) & 0xFFFFFFFFULL);
 constexpr uint32_t kHitBelow = 858993456u;                        // 4 * floor((2^30 - 1) / 5)
-constexpr uint32_t kQLimbMul = 5u << 15;                          // (L * 5 * 2^32) >> 17
 
-// Per-(column, row) shared part: D and the parity seed from the low 17 bits of X and Z.
-struct Shared {
-    uint32_t carry;   // carry out of the low 17 bits of X + Z
-    uint32_t d;       // 2 * Q * inv5
-    uint32_t q0;      // bit 0 of Q (parity contribution)
-};
+// Low 17 bits of a term at the top of a word: the sum of two of them carries out of the word, and the
+// high word of its product with A is (l * A + 11) >> 17 without a shift.
+__host__ __device__ __forceinline__ uint32_t low_bits(uint64_t term) { return (uint32_t)term << (32 - kPeriodBits); }
 
-__host__ __device__ __forceinline__ Shared shared_part(uint32_t x_lo17, uint32_t z_lo17) {
-    const uint32_t s = x_lo17 + z_lo17;
-    const uint32_t l = (s & 0x1FFFFu) ^ kXorLo;
-    const uint64_t prod = (uint64_t)l * kA32 + 11u;
-    const uint32_t q = (uint32_t)(prod >> kPeriodBits) + l * kQLimbMul;
-    return Shared{s >> kPeriodBits, q * kTwoInv5, q & 1u};
+#ifdef __CUDACC__
+// Shared part of one (column, row) of two X phases (high parts x0, x1 of the column term, low bits lo)
+// and the row's low bits zlo; zpar is bit 0 of (its high part in band 0) ^ kXorHi. Gives d = 2 Q inv5,
+// which phase of the pair can have an even first draw in even bands (`odd`: the second), and the high
+// parts, carry added, that even (xa) and odd bands (xb) test. 5 inv5 = 1 (mod 2^32), so with
+// Q = hi + 5 l', d = 2 inv5 hi + 2 l'; zpar rides in the product's high word and leaves d again. Eight
+// integer-ALU instructions (@cycles@).
+__device__ __forceinline__ void shared_part(uint32_t lo, uint32_t x0, uint32_t x1, uint32_t zlo, uint32_t zpar,
+                                            uint32_t& xa, uint32_t& xb, uint32_t& d, bool& odd) {
+    uint32_t l, c0, c1;
+    asm("{ add.cc.u32 %0, %3, %4;\n addc.u32 %1, %5, 0;\n addc.u32 %2, %6, 0; }"
+        : "=&r"(l), "=&r"(c0), "=r"(c1) : "r"(lo), "r"(zlo), "r"(x0), "r"(x1));
+    l ^= kXorLo << (32 - kPeriodBits);
+    const uint64_t prod = (uint64_t)l * kA32 + (((uint64_t)zpar << 32) | (11u << (32 - kPeriodBits)));
+    const uint32_t hi = (uint32_t)(prod >> 32);
+    d = hi * kTwoInv5 + (l * 2u - (zpar ? kTwoInv5 : 0u));
+    odd = ((hi ^ c0) & 1u) != 0;
+    xa = odd ? c1 : c0;
+    xb = odd ? c0 : c1;
 }
+#endif
 
 // Exact first-draw test of one chunk from full 64-bit terms (used by checks and fix-ups).
 __host__ __device__ __forceinline__ bool first_draw_slime(uint64_t xt, uint64_t zt_seeded) {

@@ -49,7 +49,7 @@ constexpr unsigned kFull = 0xFFFFFFFFu;
 // Row-term record of one base row for one group of up to 32 bands (matches the global table
 // written by row_terms_kernel, so a batch of 8 rows is one contiguous 1,152-byte bulk copy).
 constexpr int kRowWords = 36;
-constexpr int kRowLo = 32;      // low 17 bits of the row term (shared by all bands)
+constexpr int kRowLo = 32;      // low_bits of the row term (shared by all bands)
 constexpr int kRowValid = 33;   // bands of the group that hold this row (prefix count)
 
 // Grouped-band record: [m] high part and [32 + m] low 17 bits of the row term in band m, [64] bands holding the row.
@@ -516,7 +516,7 @@ __device__ __forceinline__ bool band_tile(BandSmem& S, const BandArgs& a, int64_
             const int64_t idx0 = (int64_t)T.u0 + (gw + k) * 32 + lane + (int64_t)T.i0 * kPeriod;
             const uint64_t x0 = idx0 < a.ncols ? a.ct[idx0] : 0;
             const uint64_t x1 = idx0 + kPeriod < a.ncols ? a.ct[idx0 + kPeriod] : 0;
-            lox[k] = (uint32_t)x0 & 0x1FFFFu;
+            lox[k] = low_bits(x0);
             xh0[k] = (uint32_t)(x0 >> kPeriodBits);
             xh1[k] = (uint32_t)(x1 >> kPeriodBits);
         }
@@ -579,12 +579,9 @@ __device__ __forceinline__ bool band_tile(BandSmem& S, const BandArgs& a, int64_
                     uint32_t xa[kGenW], xb[kGenW], dd[kGenW], sw[kGenW];
 #pragma unroll
                     for (int k = 0; k < kGenW; ++k) {
-                        const Shared sh = shared_part(lox[k], zlo);
-                        const uint32_t pi = (sh.q0 ^ xh0[k] ^ sh.carry ^ zpar) & 1u;
-                        xa[k] = (pi ? xh1[k] : xh0[k]) + sh.carry;
-                        xb[k] = (pi ? xh0[k] : xh1[k]) + sh.carry;
-                        dd[k] = sh.d;
-                        sw[k] = __ballot_sync(kFull, pi != 0);
+                        bool odd;
+                        shared_part(lox[k], xh0[k], xh1[k], zlo, zpar, xa[k], xb[k], dd[k], odd);
+                        sw[k] = __ballot_sync(kFull, odd);
                     }
                     store_plane(dst + (kGrpSw + g) * kPlaneStep, sw);
                     // Copies c and c + 1: bands m = c G + g and m + G (even copies test the phase
@@ -629,12 +626,9 @@ __device__ __forceinline__ bool band_tile(BandSmem& S, const BandArgs& a, int64_
                 uint32_t xa[kGenW], xb[kGenW], dd[kGenW], sw[kGenW];
 #pragma unroll
                 for (int k = 0; k < kGenW; ++k) {
-                    const Shared sh = shared_part(lox[k], zlo);
-                    const uint32_t pi = (sh.q0 ^ xh0[k] ^ sh.carry ^ zpar) & 1u;
-                    xa[k] = (pi ? xh1[k] : xh0[k]) + sh.carry;
-                    xb[k] = (pi ? xh0[k] : xh1[k]) + sh.carry;
-                    dd[k] = sh.d;
-                    sw[k] = __ballot_sync(kFull, pi != 0);
+                    bool odd;
+                    shared_part(lox[k], xh0[k], xh1[k], zlo, zpar, xa[k], xb[k], dd[k], odd);
+                    sw[k] = __ballot_sync(kFull, odd);
                 }
                 // Plane m of the warp's 4 words at dst + m * kWords (16-byte aligned). Every lane
                 // stores the same ballot words to the same address: no predicate, no branch.
@@ -832,7 +826,7 @@ __global__ void row_terms_kernel(uint32_t* rt, int32_t vrows_alloc, int32_t vrow
             if (j < nj && off < limit) {
                 const int32_t c = (int32_t)((int64_t)first + off);
                 const uint64_t t = (use_x_term ? x_term(c) : z_term(c)) + (uint64_t)seed;
-                out = lo ? (uint32_t)t & 0x1FFFFu : (uint32_t)(t >> kPeriodBits);
+                out = lo ? low_bits(t) : (uint32_t)(t >> kPeriodBits);
             }
         } else if (w == kValid) {
             if (kMode == kModeGrouped) {  // one group of at most 16 bands, rows increasing with j

@@ -286,13 +286,9 @@ __device__ __forceinline__ void generate_row(const BandArgs& a, const Tile& T, c
         uint32_t xa[4], xb[4], dd[4], even[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            // pi: which phase of the pair can have an even first draw in even bands.
-            const band::Shared sh = shared_part(C.lo[k], zlo);
-            const uint32_t pi = (sh.q0 ^ C.h0[k] ^ sh.carry ^ zpar) & 1u;
-            xa[k] = (pi ? C.h1[k] : C.h0[k]) + sh.carry;
-            xb[k] = (pi ? C.h0[k] : C.h1[k]) + sh.carry;
-            dd[k] = sh.d;
-            even[k] = 0x55555555u ^ (0u - pi);  // bands whose hit belongs to phase 0
+            bool odd;
+            shared_part(C.lo[k], C.h0[k], C.h1[k], zlo, zpar, xa[k], xb[k], dd[k], odd);
+            even[k] = odd ? 0xAAAAAAAAu : 0x55555555u;  // bands whose hit belongs to phase 0
         }
 #pragma unroll 2
         for (int m = (bands - 1) & ~3; m >= 0; m -= 4) {
@@ -321,7 +317,7 @@ __device__ __forceinline__ void generate_row(const BandArgs& a, const Tile& T, c
         }
     } else {
         const int G = a.groups, copies = T.copies;
-        const uint32_t all = (1u << copies) - 1u;
+        const uint32_t even_copies = 0x5555u & ((1u << copies) - 1u), odd_copies = 0xAAAAu & ((1u << copies) - 1u);
         uint32_t first[4] = {0u, 0u, 0u, 0u};  // per band: the hit belongs to phase 0
 #pragma unroll 1
         for (int g = G - 1; g >= 0; --g) {
@@ -330,12 +326,9 @@ __device__ __forceinline__ void generate_row(const BandArgs& a, const Tile& T, c
             uint32_t xa[4], xb[4], dd[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                const band::Shared sh = shared_part(C.lo[k], zlo);
-                const uint32_t pi = (sh.q0 ^ C.h0[k] ^ sh.carry ^ zpar) & 1u;
-                xa[k] = (pi ? C.h1[k] : C.h0[k]) + sh.carry;
-                xb[k] = (pi ? C.h0[k] : C.h1[k]) + sh.carry;
-                dd[k] = sh.d;
-                first[k] = (first[k] << copies) | ((0x5555u ^ (0u - pi)) & all);
+                bool odd;
+                shared_part(C.lo[k], C.h0[k], C.h1[k], zlo, zpar, xa[k], xb[k], dd[k], odd);
+                first[k] = (first[k] << copies) | (odd ? odd_copies : even_copies);
                 miss[k] <<= copies - bands;  // copies without a centre in the tile: not valid
             }
             int c = bands;
@@ -754,7 +747,7 @@ __device__ __forceinline__ bool plane_tile(PlaneSmem& S, const BandArgs& a, int6
         } else {
             const uint64_t x1 = idx0 + kPeriod < a.ncols ? a.ct[idx0 + kPeriod] : 0;
             C.absent |= (idx0 + kPeriod < a.ncols ? 0u : 1u) << (4 + k);
-            C.lo[k] = (uint32_t)x0 & 0x1FFFFu;
+            C.lo[k] = low_bits(x0);
             C.h0[k] = (uint32_t)(x0 >> kPeriodBits);
             C.h1[k] = (uint32_t)(x1 >> kPeriodBits);
         }
@@ -951,9 +944,9 @@ __global__ void __launch_bounds__(kTpb, kCtasPerSm) plane_batch_kernel(const Ban
 // 32 g + m holds base row v at input row v + offset(j), where offset(j) = j * stride, or, with grouped
 // bands, (j % P) * 2^17 + (j / P) * stride (P copies a group). Record words (0 where the row lies
 // outside the area plus halo):
-//   shared LCG   [m] high part (>> 17) of the row term in band m, [32] its low 17 bits, [33] bands
+//   shared LCG   [m] high part (>> 17) of the row term in band m, [32] its low_bits, [33] bands
 //   independent  [m] and [32 + m]: indep_hi and indep_lo of the row term in band m, [64] bands
-//   grouped      [m] high part and [32 + m] low 17 bits of the row term in band m, [64] bands
+//   grouped      [m] high part and [32 + m] low_bits of the row term in band m, [64] bands
 // "bands" is the mask of the bands that hold the row. Rows v >= vrows (padding) are zero.
 template <int kMode>
 __global__ void row_terms_kernel(uint32_t* rt, int32_t vrows_alloc, int32_t vrows, int32_t nj,
@@ -983,7 +976,7 @@ __global__ void row_terms_kernel(uint32_t* rt, int32_t vrows_alloc, int32_t vrow
                 const int32_t c = (int32_t)((int64_t)first + row);
                 const uint64_t t = (use_x_term ? x_term(c) : z_term(c)) + (uint64_t)seed;
                 if (kMode == kModeIndep) out = hi ? indep_hi(t) : indep_lo(t);
-                else out = hi ? (uint32_t)(t >> kPeriodBits) : (uint32_t)t & 0x1FFFFu;
+                else out = hi ? (uint32_t)(t >> kPeriodBits) : low_bits(t);
             }
         }
     }
