@@ -131,18 +131,16 @@ void slime_b200_set_engine(int32_t mode, int32_t band_min_threshold);
 /* The automatic engine rule as 6, 8 or 12 numbers: {band_min_threshold, band_min_periods,
  * band_fast_threshold, band_fast_periods, indep_min_threshold, indep_min_centres,
  * exact_below_threshold, exact_min_centres, grouped_min_threshold, grouped_min_width,
- * grouped_max_width, exact_wide_below_threshold}. Thresholds below exact_below_threshold (on areas
- * 4 x 2^17 chunks wide or more: below exact_wide_below_threshold; narrower areas that the grouped
- * bands take are left to them) on areas of
- * exact_min_centres centres or more use the band engines with bit-sliced exact counts (shared LCG
- * on areas band_fast_periods x 2^17 chunks wide, grouped bands from 4 x 2^17 up to
- * grouped_max_width, else independent bands) while the expected
- * number of sites stays below 1e9. Otherwise grouped bands (X phase pairs with groups of Z period
- * copies) take areas grouped_min_width .. grouped_max_width chunks wide (at most 16 x 2^17) from
- * grouped_min_threshold; the shared-LCG band engine takes areas at least
- * band_min_periods x 2^17 chunks wide from band_min_threshold, or band_fast_periods x 2^17 wide
- * from band_fast_threshold; independent bands take areas of indep_min_centres centres or more from indep_min_threshold; the
- * general scan takes the rest. Thresholds 28..222 (222 disables a branch;
+ * grouped_max_width, exact_wide_below_threshold}. The shared-LCG band engine takes areas at least
+ * band_min_periods x 2^17 chunks wide from band_min_threshold, or band_fast_periods x 2^17 wide from
+ * band_fast_threshold; grouped bands (X phase pairs x groups of Z period copies) take areas
+ * grouped_min_width .. grouped_max_width chunks wide (at most 16 x 2^17) from grouped_min_threshold,
+ * before the shared LCG. Of the others, thresholds below exact_below_threshold (on areas 2.25 x 2^17
+ * chunks wide or more: below exact_wide_below_threshold) on areas of exact_min_centres centres or more
+ * use the bit-plane kernels with exact counts (independent bands; from 2.25 x 2^17 grouped bands; from
+ * 16 x 2^17 the shared LCG) while the expected number of sites stays below 1e9. Independent bands take
+ * areas of indep_min_centres centres or more from indep_min_threshold; the general scan takes the rest.
+ * Thresholds 28..222 (222 disables a branch;
  * exact_below_threshold and exact_wide_below_threshold 0..222, 0 disables them;
  * grouped_min_threshold 28..222), periods 2..64,
  * widths >= 0. With n = 6 or 8 the numbers not given are kept. Returns 0, or -1 for a wrong count or a value out of range (nothing is changed).

@@ -37,8 +37,7 @@ bool Context::ensure_band() {
 
 // Engine choice. The band engines need a threshold >= 28 (their byte-lane bound test). The
 // shared-LCG band engine wants an area spanning two periods on one axis; the independent-band
-// engine wants enough centres to fill the GPU. Below their thresholds the exact counts of the
-// many surviving 4x4 groups dominate and the general scan is faster.
+// engine wants enough centres to fill the GPU. The general scan takes the rest.
 int32_t Context::engine_for(const SearchSpec& q) const {
     if (engine_override == 4) return kAlgoBandExact;
     if (engine_override == 5) return kAlgoIndepExact;
@@ -48,30 +47,29 @@ int32_t Context::engine_for(const SearchSpec& q) const {
     if (engine_override == 2) return kAlgoBand;
     if (engine_override == 3) return kAlgoIndep;
     if (engine_override == 6) return groups_fit ? kAlgoGrouped : kAlgoBand;
-    // The rule's numbers are measured crossovers (slime_b200/autotune.py writes them; the
-    // defaults are the B200 values). The shared LCG pays off with many periods (its work is
-    // shared by every band and phase pair) and a high threshold.
+    // The rule's numbers are measured crossovers (slime_b200/autotune.py writes them; the defaults are
+    // the B200 values).
     const int64_t w = 2 * q.rd_max + 1;
-    // Low thresholds: exact counts of every centre, while the sites stay few enough to collect
-    // (the band engines emit every site in range; the general scan gates by count on the device).
+    const bool wide = w >= kGroupedExactMinWidth, copies_fit = w <= kGroupedMaxPeriods * kP;
+    // Columns in words (bounded counts): shared LCG and grouped bands at high thresholds. Their
+    // generator is cheaper than the bit planes', and few groups of windows pass its bounds there.
+    const bool shared = (q.min_size >= band_min_threshold && w >= (int64_t)band_min_periods * kP) ||
+                        (q.min_size >= band_fast_threshold && w >= (int64_t)band_fast_periods * kP);
+    const bool grouped = q.min_size >= grouped_min_threshold && w >= grouped_min_width && w <= grouped_max_width && copies_fit;
+    // Bit planes (exact counts) below that, while the sites stay few enough to collect (the band
+    // engines emit every site in range; the general scan gates by count on the device). The generator's
+    // sharing and how full the words are decide the mode. B200, T centres/s at threshold 44: independent
+    // bands 1.60-1.68 at any width; grouped bands 1.26 / 1.64 / 1.74 / 2.22 / 3.41 at 1.5 / 2.3 / 3.1 /
+    // 4.6 / 15.3 periods; the shared LCG 1.54 / 2.43 / 2.86 at 9.2 / 15.3 / 19.1.
     constexpr double kExactMaxSites = 1e9;
-    const bool wide = w >= kGroupedExactMinPeriods * kP;
-    const bool grouped_width = w >= grouped_min_width && w <= grouped_max_width && w <= kGroupedMaxPeriods * kP;
-    // Areas one to several periods wide: X phase pairs with groups of Z period copies.
-    const bool grouped = q.min_size >= grouped_min_threshold && grouped_width;
-    if (!(grouped && !wide) && q.min_size < (wide ? exact_wide_below_threshold : exact_below_threshold) &&
+    if (!shared && !grouped && q.min_size < (wide ? exact_wide_below_threshold : exact_below_threshold) &&
         w * w >= exact_min_centres && (double)w * (double)w * tail_share(q.min_size) <= kExactMaxSites)
-        // Exact counts cost the same per centre in every mode; the generator's sharing and how full
-        // the words are decide: independent bands on narrow areas, grouped bands from 4 periods
-        // (measured on B200: 1.71 against 1.39 T/s at 4.6 periods, 1.35 against 1.39 at 3 periods), the
-        // shared LCG on the widest.
-        return w >= (int64_t)band_fast_periods * kP ? kAlgoBandExact
-               : wide && w <= grouped_max_width && w <= kGroupedMaxPeriods * kP ? kAlgoGroupedExact
-                                                                                : kAlgoIndepExact;
+        // Independent bands run the same kernels either way; counted by unions of windows they are
+        // reported as bounded.
+        return !wide ? (plane_union(q.min_size) > 1 ? kAlgoIndep : kAlgoIndepExact)
+               : copies_fit ? kAlgoGroupedExact : kAlgoBandExact;
     if (grouped) return kAlgoGrouped;
-    if ((q.min_size >= band_min_threshold && w >= (int64_t)band_min_periods * kP) ||
-        (q.min_size >= band_fast_threshold && w >= (int64_t)band_fast_periods * kP))
-        return kAlgoBand;
+    if (shared) return kAlgoBand;
     if (w * w >= indep_min_centres && q.min_size >= indep_min_threshold) return kAlgoIndep;
     return kAlgoGeneral;
 }
@@ -159,11 +157,13 @@ cudaError_t launch_band_scan(const BandArgs& a, int grid, cudaStream_t s) {
     return band_planes(band_mode(a), a.exact != 0) ? launch_plane_scan(a, grid, s) : launch_column_scan(a, grid, s);
 }
 
-// 0..3: columns in words, by mode (shared, grouped) and survivor lists; 4..7: bit planes.
+// 0..3: columns in words, by mode (shared, grouped) and survivor lists; 4..12: bit planes, by mode and
+// windows counted as one.
 int band_class(const BandArgs& a) {
     const int mode = band_mode(a);
-    if (band_planes(mode, a.exact != 0)) return mode == kBandIndep ? 4 + (a.exact ? 1 : 0) : mode == kBandGrouped ? 6 : 7;
-    return (mode == kBandGrouped ? 2 : 0) + (band_keeps_candidates(a.min_size) ? 1 : 0);
+    if (!band_planes(mode, a.exact != 0)) return (mode == kBandGrouped ? 2 : 0) + (band_keeps_candidates(a.min_size) ? 1 : 0);
+    const int joined = plane_union(a.min_size);
+    return 4 + 3 * mode + (joined == 4 ? 2 : joined - 1);
 }
 
 bool Context::scan_band(const SearchSpec& q, std::vector<Hit>& best, std::vector<uint32_t>& h,

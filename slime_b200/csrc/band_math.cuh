@@ -44,8 +44,8 @@ __host__ __device__ __forceinline__ uint32_t low_bits(uint64_t term) { return (u
 // and the row's low bits zlo; zpar is bit 0 of (its high part in band 0) ^ kXorHi. Gives d = 2 Q inv5,
 // which phase of the pair can have an even first draw in even bands (`odd`: the second), and the high
 // parts, carry added, that even (xa) and odd bands (xb) test. 5 inv5 = 1 (mod 2^32), so with
-// Q = hi + 5 l', d = 2 inv5 hi + 2 l'; zpar rides in the product's high word and leaves d again. Eight
-// integer-ALU instructions (@cycles@).
+// Q = hi + 5 l', d = 2 inv5 hi + 2 l'; zpar rides in the product's high word and leaves d again.
+// Eight integer-ALU instructions.
 __device__ __forceinline__ void shared_part(uint32_t lo, uint32_t x0, uint32_t x1, uint32_t zlo, uint32_t zpar,
                                             uint32_t& xa, uint32_t& xb, uint32_t& d, bool& odd) {
     uint32_t l, c0, c1;

@@ -67,7 +67,7 @@ constexpr int32_t kAlgoGroupedExact = 230;  // grouped bands with bit-sliced exa
 // Grouped bands hold at most this many bands; the rule uses them up to this width in periods.
 constexpr int64_t kGroupedMaxBands = 16;
 constexpr int64_t kGroupedMaxPeriods = 16;
-constexpr int64_t kGroupedExactMinPeriods = 4;  // exact counts: grouped bands from this width
+constexpr int64_t kGroupedExactMinWidth = 9LL << 15;  // exact counts: grouped bands from 2.25 periods
 
 // Band mode (band_geometry) of a band algorithm.
 inline int band_mode_of(int32_t algo) {
@@ -149,28 +149,25 @@ struct Context {
     // Engine rule (engine_for; slime_b200_set_engine_rule): the shared-LCG band engine for areas
     // at least band_min_periods periods wide from band_min_threshold, or band_fast_periods wide
     // from band_fast_threshold; independent bands for areas of indep_min_centres centres or more
-    // from indep_min_threshold; the general scan otherwise. Defaults: the rule slime_b200/
-    // autotune.py derived on B200 (slime_b200/tuning_b200.json).
-    int32_t band_min_threshold = 44;
-    int32_t band_min_periods = 15;
-    int32_t band_fast_threshold = 44;
-    int32_t band_fast_periods = 15;
+    // from indep_min_threshold; the general scan otherwise. Defaults: B200 measurements
+    // (slime_b200/tuning_b200.json).
+    int32_t band_min_threshold = 53;
+    int32_t band_min_periods = 16;
+    int32_t band_fast_threshold = 55;
+    int32_t band_fast_periods = 8;
     int32_t indep_min_threshold = 42;
     int64_t indep_min_centres = 400040001;
-    // Below exact_below_threshold, areas of exact_min_centres centres or more use the band engines
-    // with bit-sliced exact counts (shared LCG on areas band_fast_periods periods wide, else
-    // independent bands), as long as the expected number of sites stays below kExactMaxSites and the
-    // grouped bands do not take them.
-    int32_t exact_below_threshold = 51;
+    // Below exact_below_threshold (kGroupedExactMinWidth and wider: exact_wide_below_threshold), areas of
+    // exact_min_centres centres or more that neither the shared LCG nor grouped bands take use the
+    // bit-plane kernels with exact counts, as long as the expected number of sites stays below 1e9.
+    int32_t exact_below_threshold = 55;
     int64_t exact_min_centres = 400040001;
     // Grouped bands for areas grouped_min_width .. grouped_max_width chunks wide (at most
-    // kGroupedMaxPeriods periods) from grouped_min_threshold, before the shared-LCG rule.
-    int32_t grouped_min_threshold = 48;
-    // Areas kGroupedExactMinPeriods periods wide or more use exact counts below this threshold
-    // instead (their exact modes share more of the generator's work).
-    int32_t exact_wide_below_threshold = 48;
-    int64_t grouped_min_width = 300001;
-    int64_t grouped_max_width = 2000001;
+    // kGroupedMaxPeriods periods) from grouped_min_threshold.
+    int32_t grouped_min_threshold = 55;
+    int32_t exact_wide_below_threshold = 55;
+    int64_t grouped_min_width = 200001;
+    int64_t grouped_max_width = 1000001;
     int64_t last_rare = 0;             // rare redraw chunks found by the last band search
     uint32_t wait_polls = 1u << 22;    // bounded mbarrier waits of the band kernels
 

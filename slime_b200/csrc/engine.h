@@ -108,8 +108,8 @@ constexpr int kBandShared = 0, kBandIndep = 1, kBandGrouped = 2;
 BandGeom band_geometry(int64_t W, int64_t H, int mode, bool planes, int sm_count);
 
 // Two kernel families share BandArgs. scan_band.cu: a word holds 32 columns of one combo (bounded
-// counts of shared and grouped bands). scan_planes.cu: a word holds 32 combos of one column (exact
-// counts, and independent bands).
+// counts of shared and grouped bands). planes.cuh: a word holds 32 combos of one column (exact counts,
+// and independent bands).
 inline bool band_planes(int mode, bool exact) { return exact || mode == kBandIndep; }
 inline int band_mode(const BandArgs& a) { return a.indep ? kBandIndep : a.groups ? kBandGrouped : kBandShared; }
 int band_max_bands();
@@ -126,13 +126,21 @@ cudaError_t launch_column_row_terms(uint32_t* rt, int32_t vrows_alloc, int32_t v
                                     cudaStream_t s);
 cudaError_t launch_column_terms(uint64_t* ct, int32_t first, int32_t n, bool transposed, cudaStream_t s);
 
+// planes_shared.cu, planes_indep.cu, planes_grouped.cu (see run_mode in planes.cuh).
+cudaError_t run_planes_shared(int joined, const BandArgs& one, const BandArgs* args, const int64_t* prefix,
+                              int32_t nsearch, unsigned long long* head, int grid, cudaStream_t s);
+cudaError_t run_planes_indep(int joined, const BandArgs& one, const BandArgs* args, const int64_t* prefix,
+                             int32_t nsearch, unsigned long long* head, int grid, cudaStream_t s);
+cudaError_t run_planes_grouped(int joined, const BandArgs& one, const BandArgs* args, const int64_t* prefix,
+                               int32_t nsearch, unsigned long long* head, int grid, cudaStream_t s);
 int plane_tile_out_w(int mode);
 int plane_row_words(int mode);
 int plane_ctas_per_sm();
 cudaError_t plane_prepare();
 cudaError_t launch_plane_scan(const BandArgs& a, int grid, cudaStream_t s);
 cudaError_t launch_plane_batch(const BandArgs* args, const int64_t* prefix, int32_t nsearch, unsigned long long* head,
-                               int mode, bool exact, int grid, cudaStream_t s);
+                               int mode, int joined, int grid, cudaStream_t s);
+int plane_union(int min_size);  // adjacent windows counted as one at a threshold
 cudaError_t launch_plane_row_terms(uint32_t* rt, int32_t vrows_alloc, int32_t vrows, int32_t nj, int32_t row_first,
                                    int64_t row_limit, int64_t row_stride, int64_t seed, bool transposed, bool indep,
                                    int32_t groups, cudaStream_t s);
@@ -144,8 +152,8 @@ cudaError_t launch_band_terms(uint64_t* ct, uint32_t* rt, const BandGeom& g, int
 size_t band_row_table_words(const BandGeom& g);
 int band_grid(bool planes, int sm_count);
 cudaError_t launch_band_scan(const BandArgs& a, int grid, cudaStream_t s);
-// Launch classes: kernel family, band mode, and survivor lists or exact counts.
-constexpr int kBandClasses = 8;
+// Launch classes: kernel family, band mode, and survivor lists or windows counted as one.
+constexpr int kBandClasses = 13;
 int band_class(const BandArgs& a);
 // Uploads band work items of any classes (reordered by class in place) and runs them: one
 // persistent launch per class present, whose CTAs take the tiles of the class's items from a device
