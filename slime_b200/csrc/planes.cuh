@@ -19,7 +19,7 @@
 //    one count then stands for 1, 2 or 4 columns. A union that reaches the threshold is looked at by
 //    the whole warp, which counts its windows one by one.
 // What bounds it (B200): integer issue. Independent bands, radius 100,000: the generator is 19-20 ms
-// (15.9 cycles a warp test in a probe of it alone; its one wide multiply costs about five of them);
+// (13.9 cycles a warp test in a probe of it alone);
 // with the counter 27.1 ms at threshold 42, 25.0 at 44 and 23.3 at 60. Packing columns took 42.4 ms at threshold 42 and 29.3 at 60.
 // Grouped bands, radius 300,000, threshold 44: 162 against 276 ms, threshold 50 (there bounded): 135 against 183 ms.
 // Shared and grouped bands at high thresholds stay with columns in words (radius 1,250,000, threshold 60:
@@ -61,10 +61,11 @@ constexpr int row_words() { return kMode == kModeShared ? kRowWordsS : kRowWords
 template <int kMode>
 constexpr int row_valid() { return kMode == kModeShared ? 33 : 64; }
 
-// Independent bands split a term at bit 18, the low part shifted up by 14: the product's high word
-// is then state1 >> 18 and the top bit of its low word the parity of the first draw.
+// Independent bands split a term at bit 18. The low parts sit at bits 2..19 (where a double's high word
+// wants them); a row's carries the bits above, so that the sum's carry leaves the word.
 constexpr int kIndepBits = 18;
-__host__ __device__ __forceinline__ uint32_t indep_lo(uint64_t t) { return (uint32_t)t << (32 - kIndepBits); }
+__host__ __device__ __forceinline__ uint32_t indep_lo(uint64_t t) { return ((uint32_t)t & 0x3FFFFu) << 2; }
+__host__ __device__ __forceinline__ uint32_t indep_row_lo(uint64_t t) { return indep_lo(t) + 0xFFF00000u; }
 __host__ __device__ __forceinline__ uint32_t indep_hi(uint64_t t) { return (uint32_t)(t >> kIndepBits); }
 
 // Tile shape of a mode: kNW words a column (one a phase with the shared LCG), kTW input columns.
@@ -243,21 +244,23 @@ __device__ __forceinline__ void shift_test(uint32_t& w, uint32_t x, uint32_t z, 
     shift_miss(w, ((x + z) ^ kXorHi) * kMulH + d, kHitBelow);
 }
 
-// First-draw test of one chunk from split terms (independent bands: nothing is shared). With the
-// seed mix M = H * 2^18 + l and lo = l * 2^14, the product (M ^ S) * A + 11, taken times 2^14, has
-// u = state1 >> 18 in its high word and bit 17 of state1 (the parity of the first draw) in the top
-// bit of its low word. An even draw is 2 u (u mod 2^30), and it is a multiple of 10 below the
-// rejection bound iff 4 u inv5 (mod 2^32) < kHitBelow; kHitBelow < 2^31, so the parity bit is OR-ed
-// in. Eleven instructions.
+// First-draw test of one chunk from split terms (independent bands: nothing is shared). With state0 =
+// H * 2^18 + l, bits = v + H * 2 A (mod 2^31) with v = (l * A + 11) >> 17, a 53-bit product that one FP64
+// multiply-add gives exactly: d = 2^18 + l + 2^-31 stands in the words of a double, d * A / 2^17 plus
+// (3 * 2^51 - 2 A) is 3 * 2^51 + (l * A + 11.74) / 2^17, and rounding to zero leaves v in the low word (the
+// .74 never reaches the next integer). y = 2 bits inv5 is below kHitBelow and a multiple of 4 iff the
+// draw is an even multiple of 10 below the bound; rotated by 2 that is one comparison. The integer form
+// (a 32 x 32 -> 64 multiply) ran 15.8 cycles a warp test, this one 13.9.
 __device__ __forceinline__ void shift_indep(uint32_t& w, uint32_t xl, uint32_t xh, uint32_t zl, uint32_t zh) {
+    constexpr double kA = 25214903917.0;  // 0x5DEECE66D
+    static_assert(0x5DEECE66DLL == 25214903917LL, "LCG multiplier");
     uint32_t lo, hi;
     asm("{ add.cc.u32 %0, %2, %3;\n addc.u32 %1, %4, %5; }" : "=r"(lo), "=r"(hi) : "r"(xl), "r"(zl), "r"(xh), "r"(zh));
-    lo ^= indep_lo(band::kSeedXor);
+    const uint32_t high = (lo & 0xFFFFCu) ^ (0x41100000u ^ indep_lo(band::kSeedXor));  // 2^18 + l
+    const double v = __fma_rz(__hiloint2double((int)high, 8), kA / 131072.0, 6755399441055744.0 - 2.0 * kA);
     hi ^= indep_hi(band::kSeedXor);
-    const uint64_t prod = (uint64_t)lo * kA32 + (11ull << (32 - kIndepBits));
-    // u = (high word) + 5 lo + A hi, and 20 inv5 = 4 (mod 2^32).
-    const uint32_t y = (uint32_t)(prod >> 32) * (4u * kInv5) + (hi * (4u * kInv5 * kA32) + (lo << 2));
-    shift_miss(w, y | ((uint32_t)prod & 0x80000000u), kHitBelow);
+    const uint32_t y = (uint32_t)__double2loint(v) * kTwoInv5 + hi * (2u * kTwoInv5 * kA32);
+    shift_miss(w, __funnelshift_r(y, y, 2), kHitBelow / 4u);
 }
 
 // Column terms of a generator thread's four columns, and which do not exist (bit k: column k of

@@ -9,7 +9,7 @@ namespace {
 // bands, (j % P) * 2^17 + (j / P) * stride (P copies a group). Record words (0 where the row lies
 // outside the area plus halo):
 //   shared LCG   [m] high part (>> 17) of the row term in band m, [32] its low_bits, [33] bands
-//   independent  [m] and [32 + m]: indep_hi and indep_lo of the row term in band m, [64] bands
+//   independent  [m] and [32 + m]: indep_hi and indep_row_lo of the row term in band m, [64] bands
 //   grouped      [m] high part and [32 + m] low_bits of the row term in band m, [64] bands
 // "bands" is the mask of the bands that hold the row. Rows v >= vrows (padding) are zero.
 template <int kMode>
@@ -39,7 +39,7 @@ __global__ void row_terms_kernel(uint32_t* rt, int32_t vrows_alloc, int32_t vrow
             if (j < nj && row < limit) {
                 const int32_t c = (int32_t)((int64_t)first + row);
                 const uint64_t t = (use_x_term ? x_term(c) : z_term(c)) + (uint64_t)seed;
-                if (kMode == kModeIndep) out = hi ? indep_hi(t) : indep_lo(t);
+                if (kMode == kModeIndep) out = hi ? indep_hi(t) : indep_row_lo(t);
                 else out = hi ? (uint32_t)(t >> kPeriodBits) : low_bits(t);
             }
         }
