@@ -6,11 +6,18 @@
 // offset position (count_spawnable_cached_table, SlimeCore.cpp:291-331); keep the strict maximum,
 // first in (dx, dz, Y) order, starting from 0 at the site centre.
 //
-// B200 design: one CTA per site builds a 23 x 23 chunk bitmap covering all 81 windows once; a
-// precomputed table gives each slime chunk's block-column count for the window alignment
-// (o mod 16 on each axis), the chunk's place in the 21 x 21 window and the Y level, so a score is
-// a sum of table entries over the window's slime chunks. Threads split the (offset, Y) pairs and
-// a block reduction picks (max obs, first order).
+// B200 design: a precomputed table gives each slime chunk's block-column count for the window
+// alignment (o mod 16 on each axis), the chunk's place in the 21 x 21 window and the Y level, so a
+// score is a sum of table entries over the window's slime chunks.
+//  * One Y level (precise_one_kernel): the offsets of a site meet only 4 x 4 alignments, so a CTA keeps
+//    those slices of the table in shared memory, padded to 25 x 25 chunks with zeros, and a warp takes a
+//    site: it lists the slime chunks of the 23 x 23 that any offset reaches, and each lane adds up
+//    the entries of its three offsets. Per chunk that is one broadcast and three lookups a warp; a CTA
+//    per site with the table in global memory spent its time on 44 dependent steps of bit scanning a
+//    lane and eight block barriers a site. 20,000 sites: 243 -> 86 us (issue slots 56 % busy).
+//  * Several Y levels (precise_kernel): one CTA per site builds the 23 x 23 bitmap once; threads split the
+//    (offset, Y) pairs, neighbours in Y, so the table reads coalesce; a block reduction picks (max obs,
+//    first order).
 #include "engine.h"
 
 namespace slime {
@@ -132,6 +139,99 @@ __global__ void __launch_bounds__(kPreciseTpb) precise_kernel(const PreciseArgs 
     }
 }
 
+// ---- one Y level ---------------------------------------------------------------------------------
+
+constexpr int kOneTpb = 256, kOneWarps = kOneTpb / 32;
+constexpr int kSide = 23;               // chunks per axis that some offset's window reaches
+constexpr int kPad = 25;                // table slice side: a window's chunk index is -2 .. 22 + 2
+constexpr int kSlice = kPad * kPad;
+
+__global__ void __launch_bounds__(kOneTpb) precise_one_kernel(const PreciseArgs a, int chunk) {
+    __shared__ uint16_t table[16 * kSlice];         // [x alignment / 4][z alignment / 4][i + 2][j + 2]
+    __shared__ uint16_t list[kOneWarps][kSide * kSide];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int lo = a.scan_xz ? -16 : 0, hi = a.scan_xz ? 16 : 0;
+    const int side = a.scan_xz ? 9 : 1, pairs = side * side;
+    int loaded = -1;  // alignment class (both centres mod 4) of the table
+
+    for (int first = blockIdx.x * chunk; first < a.n; first += gridDim.x * chunk) {
+        const int last = min(first + chunk, a.n);
+        // Sites of one class at a time: the table's slices are its 16 alignments. Search results are all
+        // of class 0 (centres at 8 mod 16).
+        for (int done = 0; done < last - first;) {
+            int cls = 16;  // the smallest class not yet done
+            for (int s = first; s < last; ++s) {
+                const int c = (int)(a.sites[s].center_x & 3) * 4 + (int)(a.sites[s].center_z & 3);
+                if (c < cls && c >= (done ? loaded + 1 : 0)) cls = c;
+            }
+            if (cls != loaded || !done) {
+                __syncthreads();  // the previous table is no longer read
+                if (cls != loaded)
+                    for (int r = warp; r < 16 * kPad; r += kOneWarps) {  // one row of a slice a warp
+                        const int s = r / kPad, i = r % kPad - 2, j = lane - 2;
+                        const int ax = (s >> 2) * 4 + (cls >> 2), az = (s & 3) * 4 + (cls & 3);
+                        if (lane < kPad)
+                            table[r * kPad + lane] =
+                                i >= 0 && i < 21 && j >= 0 && j < 21 ? a.weights[(ax * 16 + az) * 441 + i * 21 + j] : 0;
+                    }
+                __syncthreads();
+                loaded = cls;
+            }
+            for (int s = first; s < last; ++s) {
+                const int64_t bx = a.sites[s].center_x, bz = a.sites[s].center_z;
+                if ((int)(bx & 3) * 4 + (int)(bz & 3) != cls) continue;
+                const bool mine = done++ % kOneWarps == warp;
+                if (!mine) continue;
+                const int64_t ux0 = floor_div16(bx + lo) - 10, uz0 = floor_div16(bz + lo) - 10;
+                const int nx = (int)(floor_div16(bx + hi) + 10 - ux0 + 1);
+                const int nz = (int)(floor_div16(bz + hi) + 10 - uz0 + 1);
+                // Slime chunks (i, j) as i * kPad + j: lane = j, one i at a time.
+                const uint64_t xs = x_term((int32_t)(ux0 + lane)), zs = z_term((int32_t)(uz0 + lane)) + (uint64_t)a.seed;
+                int n = 0;
+                __syncwarp();
+                for (int i = 0; i < nx; ++i) {
+                    const bool hit = slime_from_terms(__shfl_sync(0xFFFFFFFFu, xs, i), zs) && lane < nz;
+                    const unsigned m = __ballot_sync(0xFFFFFFFFu, hit);
+                    if (hit) list[warp][n + __popc(m & ((1u << lane) - 1u))] = (uint16_t)(i * kPad + lane);
+                    n += __popc(m);
+                }
+                __syncwarp();
+                // This lane's offsets p = lane, lane + 32, lane + 64: first table entry of chunk (0, 0).
+                int base[3], obs[3] = {0, 0, 0};
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    const int p = min(lane + 32 * k, pairs - 1);
+                    const int64_t ox = bx + lo + (p / side) * 4, oz = bz + lo + (p % side) * 4;
+                    const int wx = (int)(floor_div16(ox) - 10 - ux0), wz = (int)(floor_div16(oz) - 10 - uz0);
+                    base[k] = (int)((((ox & 15) >> 2) * 4 + ((oz & 15) >> 2)) * kSlice) + (2 - wx) * kPad + 2 - wz;
+                }
+#pragma unroll 4
+                for (int c = 0; c < n; ++c) {
+                    const int at = list[warp][c];
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) obs[k] += table[base[k] + at];
+                }
+                int best = -1, order = 0x7FFFFFFF;
+#pragma unroll
+                for (int k = 0; k < 3; ++k)
+                    if (lane + 32 * k < pairs && obs[k] > best) {  // offsets ascend: the first maximum wins
+                        best = obs[k];
+                        order = lane + 32 * k;
+                    }
+                const int top = __reduce_max_sync(0xFFFFFFFFu, best);
+                const int off = __reduce_min_sync(0xFFFFFFFFu, best == top ? order : 0x7FFFFFFF);
+                if (lane == 0) {
+                    ExtChunkResult& r = a.sites[s];
+                    const int y = top > 0 ? a.y_values[0] : a.platform_y;
+                    r.obs_count = a.pack_y ? (int32_t)((uint32_t)top | ((uint32_t)(y + 1024) << 20)) : top;
+                    r.afk_x = (int32_t)(top > 0 ? bx + lo + (off / side) * 4 : bx);
+                    r.afk_z = (int32_t)(top > 0 ? bz + lo + (off % side) * 4 : bz);
+                }
+            }
+        }
+    }
+}
+
 }  // namespace
 
 cudaError_t launch_weight_table(uint16_t* weights, const int16_t* outer, const int16_t* inner,
@@ -144,6 +244,17 @@ cudaError_t launch_weight_table(uint16_t* weights, const int16_t* outer, const i
 
 cudaError_t launch_precise(const PreciseArgs& a, cudaStream_t s) {
     if (a.n <= 0) return cudaSuccess;
+    if (a.y_count == 1) {
+        // Sites per CTA and round: an even share of one wave, whole rounds of the CTA's warps from one
+        // round on, and at most 256 (each thread looks at all of a chunk's alignments).
+        constexpr int kCtas = 148 * 4;
+        int chunk = (a.n + kCtas - 1) / kCtas;
+        if (chunk > kOneWarps) chunk = (chunk + kOneWarps - 1) / kOneWarps * kOneWarps;
+        if (chunk > 256) chunk = 256;
+        const int grid = (a.n + chunk - 1) / chunk;
+        precise_one_kernel<<<grid < kCtas ? grid : kCtas, kOneTpb, 0, s>>>(a, chunk);
+        return cudaGetLastError();
+    }
     const int grid = a.n < 148 * 16 ? a.n : 148 * 16;
     precise_kernel<<<grid, kPreciseTpb, 0, s>>>(a);
     return cudaGetLastError();
