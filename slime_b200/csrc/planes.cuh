@@ -333,6 +333,8 @@ __device__ __forceinline__ void generate_row(const BandArgs& a, const Tile& T, c
     } else {
         const int G = T.groups, copies = T.copies;
         const uint32_t even_copies = 0x5555u & ((1u << copies) - 1u), odd_copies = 0xAAAAu & ((1u << copies) - 1u);
+        // Shifts by a group's copies as multiplies: the integer ALU is the busy pipe.
+        const uint32_t step = 1u << copies, skip = 1u << (copies - bands);
         uint32_t first[4] = {0u, 0u, 0u, 0u};  // per band: the hit belongs to phase 0
 #pragma unroll 1
         for (int g = G - 1; g >= 0; --g) {
@@ -343,8 +345,8 @@ __device__ __forceinline__ void generate_row(const BandArgs& a, const Tile& T, c
             for (int k = 0; k < 4; ++k) {
                 bool odd;
                 shared_part(C.lo[k], C.h0[k], C.h1[k], zlo, zpar, xa[k], xb[k], dd[k], odd);
-                first[k] = (first[k] << copies) | (odd ? odd_copies : even_copies);
-                miss[k] <<= copies - bands;  // copies without a centre in the tile: not valid
+                first[k] = first[k] * step + (odd ? odd_copies : even_copies);
+                miss[k] *= skip;  // copies without a centre in the tile: not valid
             }
             int c = bands;
             if (c & 1) {
