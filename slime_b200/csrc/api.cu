@@ -234,14 +234,9 @@ bool Context::scan_general(const SearchSpec& q, std::vector<Hit>& best, std::vec
     const int band_h = general_band_rows(width, height, sm_count);
     const uint64_t cap = hits.count - kScanHeader;
     Hit* const first_hits = reinterpret_cast<Hit*>((char*)pinned + kScanHeaderBytes);
-    const double area = (double)width * (double)height;
-
-    // Materialise only counts that keep the expected emission well inside the buffer; the exact
-    // histogram decides afterwards whether a lower gate is needed (second pass).
-    int emit_min = q.min_size;
-    while (emit_min < q.max_size && area * tail_share(emit_min) > (double)cap / 8.0 &&
-           area * tail_share(emit_min + 1) >= 4.0 * q.max_results)
-        ++emit_min;
+    // Counts below the gate are only histogrammed; the exact histogram decides afterwards whether a
+    // lower gate is needed (second pass).
+    int emit_min = emission_gate(q, q.max_results);
 
     for (int pass = 0; pass < 3; ++pass) {
         best.clear();

@@ -230,18 +230,12 @@ bool Context::scan_band(const SearchSpec& q, std::vector<Hit>& best, std::vector
     const int grid = band_grid(G.planes, sm_count);
     const uint64_t cap = hits.count;
     // Count histogram on the device (first-draw counts of every centre in range, corrected for
-    // rare chunks by the fix-up) and an emission gate: only centres whose count reaches emit_min
-    // are sent to the host, chosen so that the expected emission stays well inside the buffer but
-    // covers max_results several times; if it falls short, the scan runs again with the exact
-    // gate the histogram gives.
+    // rare chunks by the fix-up) and an emission gate (emission_gate); if it falls short, the scan runs
+    // again with the exact gate the histogram gives.
     if ((e = hist.reserve(2 * kHistBins)) != cudaSuccess) { set_error("alloc", e); return false; }
     unsigned int* dhist = hist.ptr;
     int* ddelta = reinterpret_cast<int*>(hist.ptr + kHistBins);
-    const double area = (double)W * (double)H;
-    int32_t emit_min = q.min_size;
-    while (emit_min < q.max_size && area * tail_share(emit_min) > (double)cap / 8.0 &&
-           area * tail_share(emit_min + 1) >= 4.0 * q.max_results)
-        ++emit_min;
+    int32_t emit_min = emission_gate(q, q.max_results);
 
     for (int pass = 0; pass < 3; ++pass) {
         best.clear();

@@ -239,6 +239,7 @@ void release_biome();
 // Sizing of per-search slices (batch.cu): the share of centres a threshold keeps in a window of
 // independent p = 0.1 cells, and the share of chunks that are rare redraw chunks.
 double tail_share(int min_size);
+int32_t emission_gate(const SearchSpec& q, int64_t ranked);
 double rare_share();
 
 }  // namespace slime

@@ -99,14 +99,9 @@ void plan_job(Job& j, const Context& c) {
     const int64_t W = 2 * q.rd_max + 1;
     const int32_t algo = c.engine_for(q);
     const double centres = (double)W * (double)W;
-    // Emission gate, as the single search chooses it: the smallest count whose expected number of
-    // centres fits an eighth of the largest slice while still covering the ranked results
-    // (biome requests keep more, as the single search does) four times over.
+    // Emission gate, as the single search chooses it (biome requests keep more, as there).
     const int64_t want = (q.biome_flags & 3) ? 2LL * q.max_results + 1024 : (int64_t)q.max_results;
-    int32_t emit = q.min_size;
-    while (emit < q.max_size && centres * tail_share(emit) > (double)kServerHitCap / 8.0 &&
-           centres * tail_share(emit + 1) >= 4.0 * (double)want)
-        ++emit;
+    const int32_t emit = emission_gate(q, want);
     j.emit_min = emit;
     const double expect = centres * tail_share(emit);
     j.exact = algo_exact(algo);
