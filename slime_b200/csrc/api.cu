@@ -126,7 +126,7 @@ bool Context::ensure_y_tables() {
     cudaError_t e;
     if ((e = y_values.reserve(count)) != cudaSuccess || (e = outer.reserve(out.size())) != cudaSuccess ||
         (e = inner.reserve(in.size())) != cudaSuccess ||
-        (e = weights.reserve((size_t)16 * 16 * 441 * count)) != cudaSuccess) {
+        (e = weights.reserve(precise_weights(count))) != cudaSuccess) {
         set_error("y tables", e);
         return false;
     }

@@ -43,12 +43,14 @@ struct PreciseArgs {
     int32_t scan_xz;
     int32_t y_count;           // Y levels scored (1 when Y scan is off)
     const int32_t* y_values;   // y_count
-    const uint16_t* weights;   // [16][16][21][21][y_count] block columns per (alignment, chunk, y)
+    const uint16_t* weights;   // block columns per (alignment, chunk, y): see weight_table_kernel
     int32_t platform_y;
     int32_t pack_y;            // obs_count = obs | (y + 1024) << 20
 };
 cudaError_t launch_precise(const PreciseArgs& a, cudaStream_t s);
 
+// Entries of the weight table for y_count Y levels.
+__host__ __device__ size_t precise_weights(int32_t y_count);
 // Weight table for precise scoring from per-Y outer/inner radius tables ([y][257], -1 = none).
 cudaError_t launch_weight_table(uint16_t* weights, const int16_t* outer, const int16_t* inner,
                                 int32_t y_count, cudaStream_t s);

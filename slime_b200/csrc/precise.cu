@@ -30,18 +30,35 @@ __device__ __forceinline__ int64_t floor_div16(int64_t v) { return v >> 4; }
 
 __device__ __forceinline__ int interval_len(int a, int b) { return b >= a ? b - a + 1 : 0; }
 
-// weights[(((ax * 16 + az) * 21 + i) * 21 + j) * y_count + yi]
+// One Y level: weights[(ax * 16 + az) * kSlice + (i + 2) * kPad + j + 2], zero outside the window (a chunk
+// that only other offsets reach has index -2 .. 22) and up to the slice's 16-byte multiple.
+constexpr int kPad = 25;
+constexpr int kSlice = (kPad * kPad + 7) / 8 * 8;
+// Several: weights[(((ax * 16 + az) * 21 + i) * 21 + j) * y_count + yi].
 __global__ void weight_table_kernel(uint16_t* weights, const int16_t* outer, const int16_t* inner,
                                     int32_t y_count) {
-    const int64_t total = 16LL * 16 * 21 * 21 * y_count;
+    const int64_t total = (int64_t)precise_weights(y_count);
     for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
          e += (int64_t)gridDim.x * blockDim.x) {
-        const int yi = (int)(e % y_count);
-        int64_t rest = e / y_count;
-        const int j = (int)(rest % 21); rest /= 21;
-        const int i = (int)(rest % 21); rest /= 21;
-        const int az = (int)(rest % 16);
-        const int ax = (int)(rest / 16);
+        int yi = 0, i, j, ax, az;
+        if (y_count == 1) {
+            const int slice = (int)(e / kSlice), at = (int)(e % kSlice);
+            i = at / kPad - 2;
+            j = at % kPad - 2;
+            ax = slice / 16;
+            az = slice % 16;
+            if (i < 0 || i > 20 || j < 0 || j > 20) {
+                weights[e] = 0;
+                continue;
+            }
+        } else {
+            yi = (int)(e % y_count);
+            int64_t rest = e / y_count;
+            j = (int)(rest % 21); rest /= 21;
+            i = (int)(rest % 21); rest /= 21;
+            az = (int)(rest % 16);
+            ax = (int)(rest / 16);
+        }
         // Block offsets of the chunk relative to the scored position.
         const int rx0 = (i - 10) * 16 - ax, rz0 = (j - 10) * 16 - az;
         const int x0 = max(-128, rx0), x1 = min(128, rx0 + 15);
@@ -143,11 +160,9 @@ __global__ void __launch_bounds__(kPreciseTpb) precise_kernel(const PreciseArgs 
 
 constexpr int kOneTpb = 256, kOneWarps = kOneTpb / 32;
 constexpr int kSide = 23;               // chunks per axis that some offset's window reaches
-constexpr int kPad = 25;                // table slice side: a window's chunk index is -2 .. 22 + 2
-constexpr int kSlice = kPad * kPad;
 
 __global__ void __launch_bounds__(kOneTpb) precise_one_kernel(const PreciseArgs a, int chunk) {
-    __shared__ uint16_t table[16 * kSlice];         // [x alignment / 4][z alignment / 4][i + 2][j + 2]
+    __shared__ __align__(16) uint16_t table[16 * kSlice];  // [x alignment / 4][z alignment / 4][i + 2][j + 2]
     __shared__ uint16_t list[kOneWarps][kSide * kSide];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int lo = a.scan_xz ? -16 : 0, hi = a.scan_xz ? 16 : 0;
@@ -167,12 +182,10 @@ __global__ void __launch_bounds__(kOneTpb) precise_one_kernel(const PreciseArgs 
             if (cls != loaded || !done) {
                 __syncthreads();  // the previous table is no longer read
                 if (cls != loaded)
-                    for (int r = warp; r < 16 * kPad; r += kOneWarps) {  // one row of a slice a warp
-                        const int s = r / kPad, i = r % kPad - 2, j = lane - 2;
-                        const int ax = (s >> 2) * 4 + (cls >> 2), az = (s & 3) * 4 + (cls & 3);
-                        if (lane < kPad)
-                            table[r * kPad + lane] =
-                                i >= 0 && i < 21 && j >= 0 && j < 21 ? a.weights[(ax * 16 + az) * 441 + i * 21 + j] : 0;
+                    for (int e = tid; e < 16 * kSlice / 8; e += kOneTpb) {
+                        const int s = e / (kSlice / 8), ax = (s >> 2) * 4 + (cls >> 2), az = (s & 3) * 4 + (cls & 3);
+                        reinterpret_cast<uint4*>(table)[e] =
+                            reinterpret_cast<const uint4*>(a.weights + (ax * 16 + az) * kSlice)[e % (kSlice / 8)];
                     }
                 __syncthreads();
                 loaded = cls;
@@ -234,9 +247,13 @@ __global__ void __launch_bounds__(kOneTpb) precise_one_kernel(const PreciseArgs 
 
 }  // namespace
 
+__host__ __device__ size_t precise_weights(int32_t y_count) {
+    return 16 * 16 * (size_t)(y_count == 1 ? kSlice : 21 * 21 * (size_t)y_count);
+}
+
 cudaError_t launch_weight_table(uint16_t* weights, const int16_t* outer, const int16_t* inner,
                                 int32_t y_count, cudaStream_t s) {
-    const int64_t total = 16LL * 16 * 21 * 21 * y_count;
+    const int64_t total = (int64_t)precise_weights(y_count);
     const int blocks = (int)((total + 255) / 256 < 4096 ? (total + 255) / 256 : 4096);
     weight_table_kernel<<<blocks, 256, 0, s>>>(weights, outer, inner, y_count);
     return cudaGetLastError();
