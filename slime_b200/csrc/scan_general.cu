@@ -9,8 +9,8 @@
 // adder of two LOP3 adds 32 centres' bits): the first of its rows in full, the others by sliding down a
 // row (17 cells enter, 17 leave). Term tables are not needed: a patch computes its own.
 // The scan is latency-bound on small areas and issue-bound on large ones; it replaces a rolling-square
-// scan that ran 80 barriers a tile. B200, kernel time: radius 100 63 -> 8.5 us, radius 2,000
-// (threshold 40) 131 -> 47 us, radius 9,001 (threshold 44, annulus) 1,150 -> 440 us.
+// scan that ran 80 barriers a tile. B200, kernel time: radius 100 63 -> 9 us, radius 2,000
+// (threshold 40) 131 -> 35 us, radius 9,001 (threshold 44, annulus) 1,150 -> 440 us.
 #include <cmath>
 
 #include "engine.h"
@@ -25,6 +25,7 @@ constexpr int kWords = 8;               // words of a patch row
 constexpr int kOutW = kWords * 32 - 16;
 constexpr int kStride = kWords + 1;     // and a zero word: counting reads the next word
 constexpr int kMaxRows = 128;           // centre rows of a patch
+constexpr int kListCap = 1024;          // hits a CTA collects; more go out one by one
 
 // ---- bit-sliced counts: bit j of every word belongs to centre (or column) j ----------------------
 
@@ -255,8 +256,26 @@ __device__ __forceinline__ bool first_draw(uint32_t xl, uint32_t xh, uint32_t zl
 __global__ void __launch_bounds__(kTpb, 2) general_scan_kernel(const ScanArgs a) {
     __shared__ uint32_t rows[(kMaxRows + 16) * kStride];
     __shared__ unsigned int hist_s[kHistBins];
+    __shared__ Hit list[kListCap];
+    __shared__ unsigned int listed;
+    __shared__ unsigned long long list_at;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (int i = tid; i < kHistBins; i += kTpb) hist_s[i] = 0;
+    if (tid == 0) listed = 0;
+    __syncthreads();
+    // The CTA's hits go out together: reserving room for each cost its warp a round trip to L2.
+    auto flush = [&] {
+        const unsigned n = min(listed, (unsigned)kListCap);
+        __syncthreads();
+        if (tid == 0) {
+            list_at = atomicAdd(a.emitted, (unsigned long long)n);
+            listed = 0;
+        }
+        __syncthreads();
+        for (unsigned i = tid; i < n; i += kTpb)
+            if (list_at + i < a.cap) a.out[list_at + i] = list[i];
+        __syncthreads();
+    };
 
     const int64_t tiles = (int64_t)a.tiles_x * a.tiles_z;
     for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
@@ -280,6 +299,7 @@ __global__ void __launch_bounds__(kTpb, 2) general_scan_kernel(const ScanArgs a)
             xh[k] = hi_part(xt);
         }
         __syncthreads();  // the previous patch's rows are no longer read
+        if (listed > (unsigned)kListCap / 2) flush();
         for (int r = warp; r < out_h + 16; r += kWarps) {
             const uint64_t zt = z_term((int32_t)((int64_t)a.area_z0 + z_base - 8 + r)) + (uint64_t)a.seed;
             const uint32_t zl = lo_part(zt), zh = hi_part(zt);
@@ -327,12 +347,14 @@ __global__ void __launch_bounds__(kTpb, 2) general_scan_kernel(const ScanArgs a)
                     }
                     atomicAdd(&hist_s[count], 1u);
                     if (count < a.emit_min) continue;
-                    const unsigned mk = __activemask();
-                    const int leader = __ffs(mk) - 1;
-                    unsigned long long pos = 0;
-                    if (lane == leader) pos = atomicAdd(a.emitted, (unsigned long long)__popc(mk));
-                    pos = __shfl_sync(mk, pos, leader) + __popc(mk & ((1u << lane) - 1u));
-                    if (pos < a.cap) a.out[pos] = Hit{count, cx, cz};
+                    const Hit hit{count, cx, cz};
+                    const unsigned n = atomicAdd(&listed, 1u);
+                    if (n < (unsigned)kListCap) {
+                        list[n] = hit;
+                    } else {
+                        const unsigned long long pos = atomicAdd(a.emitted, 1ull);
+                        if (pos < a.cap) a.out[pos] = hit;
+                    }
                 }
             };
             bs_window_counts(R, Rn, cnt);
@@ -352,6 +374,7 @@ __global__ void __launch_bounds__(kTpb, 2) general_scan_kernel(const ScanArgs a)
         }
     }
     __syncthreads();
+    if (listed) flush();
     for (int i = tid; i < kHistBins; i += kTpb)
         if (hist_s[i]) atomicAdd(&a.hist[i], hist_s[i]);
 }
