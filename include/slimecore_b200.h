@@ -121,11 +121,13 @@ int64_t slime_b200_last_rare_chunks(void);
 /* Engine selection: mode 0 automatic, 1 always the general scan, 2 the shared-LCG band engine,
  * 3 the independent-band engine and 6 the grouped-band engine whenever the threshold allows it
  * (min_size >= 28), 4 / 5 / 7 the shared-LCG / independent-band / grouped-band engine with
- * bit-sliced exact counts (any threshold).
+ * bit-sliced counts of every centre (any threshold). Grouped modes wider than 16 x 2^17 chunks run as the
+ * shared LCG.
  * `band_min_threshold` (28..221, other values keep the current one) is the smallest threshold
  * automatic mode sends to the shared-LCG band engine. Results are identical either way; only
  * speed differs. get_gpu_v1_algorithm() reports 100 (general), 200 (band), 300 (independent
- * bands), 220 (grouped bands), or 210 / 310 / 230 (their exact-count modes) for the last search. */
+ * bands), 220 (grouped bands), or 210 / 310 / 230 (their bit-sliced forms; independent bands are
+ * bit-sliced in either form) for the last search. */
 void slime_b200_set_engine(int32_t mode, int32_t band_min_threshold);
 
 /* The automatic engine rule as 6, 8 or 12 numbers: {band_min_threshold, band_min_periods,
@@ -237,8 +239,8 @@ typedef struct SlimeBatchRequest {
 } SlimeBatchRequest;
 
 /* Runs n searches as one batch (each with its own biome exclusion, as slime_b200_search_biome).
- * Searches with min_size >= 28 share one persistent launch of the independent-band kernel whose CTAs take the tiles of all of them from one device queue; the
- * others (and any whose sites would not fit the batch's pool) run one by one. Request i writes
+ * Searches with min_size >= 28 share persistent launches of the band kernels, one for each band mode
+ * and counter, whose CTAs take the tiles of all its searches from one device queue; the others (and any whose sites would not fit the batch's pool) run one by one. Request i writes
  * min(total_i, max_results_i) ranked results at results + (max_results_0 + ... +
  * max_results_{i-1}) and its total to totals[i], exactly as the single search would; totals[i]
  * is -1 when request i's arguments are invalid. Returns 0, or -1 on a CUDA failure or a null

@@ -4,18 +4,18 @@
 
 For each (radius, threshold) point of a grid the search is timed with every engine that applies
 (the general scan, independent bands, grouped bands where the area spans a period, and the
-shared-LCG band engine where it spans two, the shared-LCG and independent-band engines also with
-bit-sliced exact counts at low thresholds), forced through slime_b200_set_engine; every engine
-must return the same total and the same ranked sites. From the timings it derives the eleven
+shared-LCG band engine where it spans two, all three also as bit planes), forced through slime_b200_set_engine; every engine
+must return the same total and the same ranked sites. From the timings it derives the twelve
 numbers of slime_b200_set_engine_rule:
 
   band_min_threshold, band_min_periods   shared LCG from this threshold on areas this many
   band_fast_threshold, band_fast_periods 2^17-chunk periods wide (two branches of the rule)
   indep_min_threshold, indep_min_centres independent bands instead of the general scan
-  exact_below_threshold, exact_min_centres  exact counts below this threshold on areas this large
+  exact_below_threshold, exact_min_centres  bit planes below this threshold on areas this large, where
+                                         neither of the other band branches applies
   grouped_min_threshold, grouped_min_width, grouped_max_width
                                          grouped bands from this threshold on areas this wide
-  exact_wide_below_threshold             exact counts below this threshold on areas 4+ periods wide
+  exact_wide_below_threshold             bit planes below this threshold on areas 2.25+ periods wide
 
 and writes them with the raw timings to a JSON file. SlimeCoreB200 applies that file when it
 loads the library. The general scan's rate does not depend on the area once it fills the GPU, so
@@ -49,8 +49,7 @@ def _time(core, mode, radius, thr, reps=2):
 
 
 GROUPED_MAX_PERIODS = 16  # grouped bands hold at most 16 period copies
-GROUPED_EXACT_MIN_PERIODS = 4  # the library's width from which exact counts may run as grouped bands
-EXACT_MAX_THRESHOLD = 50  # the exact modes are timed up to here (their cost does not depend on it)
+GROUPED_EXACT_MIN_WIDTH = 9 << 15  # the library's width from which bit planes run as grouped bands
 
 
 def measure(core, quick=False):
@@ -66,9 +65,8 @@ def measure(core, quick=False):
             if thr >= 42 or r <= 100_000:
                 engines += [("indep", 3)] + ([("band", 2)] if w >= 2 * PERIOD else [])
                 engines += [("grouped", 6)] if PERIOD < w <= GROUPED_MAX_PERIODS * PERIOD else []
-            if thr <= EXACT_MAX_THRESHOLD:
-                engines += [("indep_exact", 5)] + ([("band_exact", 4)] if w >= 2 * PERIOD else [])
-                engines += [("grouped_exact", 7)] if PERIOD < w <= GROUPED_MAX_PERIODS * PERIOD else []
+            engines += [("indep_exact", 5)] + ([("band_exact", 4)] if w >= 2 * PERIOD else [])
+            engines += [("grouped_exact", 7)] if PERIOD < w <= GROUPED_MAX_PERIODS * PERIOD else []
             if r <= 100_000:
                 engines.insert(0, ("general", 1))
             for name, mode in engines:
@@ -89,6 +87,21 @@ def measure(core, quick=False):
             rows.append(point)
     core.lib.slime_b200_set_engine(0, 0)
     return rows
+
+
+def planes_time(p):
+    """Time of the bit planes in the mode that the library picks for the point's width; None if not timed."""
+    w = 2 * p["radius"] + 1
+    if w >= GROUPED_EXACT_MIN_WIDTH:
+        for k in ("grouped_exact_s", "band_exact_s"):
+            if k in p:
+                return p[k]
+    return p.get("indep_exact_s")
+
+
+def planes_win(p):
+    """Against the other branches of the rule (independent bands are the same kernels in both of theirs)."""
+    return planes_time(p) < min(p[k] for k in ("general_s", "band_s", "grouped_s") if k in p)
 
 
 def derive(rows):
@@ -115,9 +128,7 @@ def derive(rows):
     indep_min_threshold = max(indep_thr.values())
     wins = [r for r, t in indep_thr.items() if t <= indep_min_threshold]
     indep_min_centres = (2 * min(wins) + 1) ** 2 if wins else 1 << 62
-    band_thr = {r: min_winning_thr(pts, "band_s", "indep_s") for r, pts in by_r.items()
-                if any("band_s" in p for p in pts)}
-    cands = sorted({(t, (2 * r + 1) // PERIOD) for r, t in band_thr.items()} | {(222, 64)})
+    cands = sorted({(p["threshold"], (2 * p["radius"] + 1) // PERIOD) for p in rows if "band_s" in p} | {(222, 64)})
     widths = sorted({2 * p["radius"] + 1 for p in rows if "grouped_s" in p})
     g_cands = [(t, lo, hi) for t in sorted({p["threshold"] for p in rows} | {222})
                for lo in widths for hi in widths if lo <= hi] or [(222, 1 << 40, 0)]
@@ -126,16 +137,16 @@ def derive(rows):
         total = 0.0
         for p in rows:
             w = 2 * p["radius"] + 1
-            best = min(p[k] for k in ("general_s", "indep_s", "band_s", "grouped_s") if k in p)
+            planes = planes_time(p)
+            best = min([p[k] for k in ("general_s", "indep_s", "band_s", "grouped_s") if k in p] + ([planes] if planes else []))
             thr = p["threshold"]
             if "grouped_s" in p and thr >= g[0] and g[1] <= w <= g[2]:
                 t_rule = p["grouped_s"]
             elif "band_s" in p and any(thr >= t and w >= n * PERIOD for t, n in (a, b)):
                 t_rule = p["band_s"]
-            elif w * w >= indep_min_centres and thr >= indep_min_threshold:
-                t_rule = p["indep_s"]
             else:
-                t_rule = p["general_s"]
+                t_rule = p["indep_s"] if w * w >= indep_min_centres and thr >= indep_min_threshold else p["general_s"]
+                t_rule = min(t_rule, planes or t_rule)
             total += t_rule / best
         return total
 
@@ -150,28 +161,21 @@ def derive(rows):
 
 
 def derive_exact(rows):
-    """exact_below_threshold: the exact modes take every threshold below it on the areas where
-    they win -- one above the highest threshold at which the best exact mode still beats every
-    other engine on all areas of at least exact_min_centres centres, the smallest measured area
-    where it wins at the lowest threshold."""
-    def exact_best(p):
-        return min(p[k] for k in ("indep_exact_s", "band_exact_s", "grouped_exact_s") if k in p)
-
-    def other_best(p):
-        return min(p[k] for k in ("general_s", "indep_s", "band_s", "grouped_s") if k in p)
-
+    """exact_below_threshold: one above the highest threshold at which the bit planes still beat every
+    other branch on all areas of at least exact_min_centres centres, the smallest measured area where
+    they win at the lowest threshold."""
     pts = [p for p in rows if "indep_exact_s" in p]
     if not pts:
         return [0, 1 << 62]
     lowest = min(p["threshold"] for p in pts)
-    winners = sorted(p["centres"] for p in pts if p["threshold"] == lowest and exact_best(p) < other_best(p))
+    winners = sorted(p["centres"] for p in pts if p["threshold"] == lowest and planes_win(p))
     if not winners:
         return [0, 1 << 62]
     min_centres = winners[0]
     below = 0
     for thr in sorted({p["threshold"] for p in pts}):
         big = [p for p in pts if p["threshold"] == thr and p["centres"] >= min_centres]
-        if big and all(exact_best(p) < other_best(p) for p in big):
+        if big and all(planes_win(p) for p in big):
             below = thr + 1
         else:
             break
@@ -179,19 +183,13 @@ def derive_exact(rows):
 
 
 def derive_exact_wide(rows):
-    """exact_wide_below_threshold: one above the highest threshold up to which the best exact mode
-    beats every other engine on every measured area at least GROUPED_EXACT_MIN_PERIODS wide."""
-    def exact_best(p):
-        return min(p[k] for k in ("indep_exact_s", "band_exact_s", "grouped_exact_s") if k in p)
-
-    def other_best(p):
-        return min(p[k] for k in ("general_s", "indep_s", "band_s", "grouped_s") if k in p)
-
-    pts = [p for p in rows if "indep_exact_s" in p and 2 * p["radius"] + 1 >= GROUPED_EXACT_MIN_PERIODS * PERIOD]
+    """exact_wide_below_threshold: one above the highest threshold up to which the bit planes beat
+    every other branch on every measured area at least GROUPED_EXACT_MIN_WIDTH wide."""
+    pts = [p for p in rows if "indep_exact_s" in p and 2 * p["radius"] + 1 >= GROUPED_EXACT_MIN_WIDTH]
     below = 0
     for thr in sorted({p["threshold"] for p in pts}):
         at = [p for p in pts if p["threshold"] == thr]
-        if all(exact_best(p) < other_best(p) for p in at):
+        if all(planes_win(p) for p in at):
             below = thr + 1
         else:
             break

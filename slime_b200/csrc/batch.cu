@@ -1,11 +1,11 @@
-// batch.cu -- many searches in one persistent launch of the independent-band kernel.
+// batch.cu -- many searches in persistent launches of the band kernels, one launch a class (band_class).
 //
 // No reference counterpart: the reference runs one search per call. Searches whose threshold
 // the band kernel's byte-lane bound accepts (min_size >= 28) and whose expected site count fits
-// the batch's hit pool are tiled together; one launch of band_batch_kernel takes their tiles
+// the batch's hit pool are tiled together; each class's launch takes its searches' tiles
 // from a device queue, so small and large areas share the GPU with no per-search tail. Term
 // tables, rare-chunk scans, filters and fix-ups of all searches are queued on the library stream
-// around that launch; ranking and precise scoring then follow per search on the host, exactly as
+// around those launches; ranking and precise scoring then follow per search on the host, exactly as
 // for a single search. Every other request runs through the single-search path.
 #include <algorithm>
 #include <cmath>
@@ -53,7 +53,7 @@ namespace {
 struct Planned {
     int32_t idx;          // request index
     BandGeom g;
-    bool exact;  // bit-sliced exact counts
+    bool exact;  // bit planes
     int32_t area_x0, area_z0;
     size_t ct_off, rt_off, hit_off, rare_off;
     uint64_t hit_cap;

@@ -58,16 +58,16 @@ constexpr int64_t kNeedMoreSites = -3;  // finish(): the biome exclusion needs m
 constexpr int32_t kAlgoGeneral = 100;
 constexpr int32_t kAlgoBand = 200;
 constexpr int32_t kAlgoIndep = 300;
-// The band engines with bit-sliced exact counts of every centre (low thresholds).
+// The band engines as bit planes (planes.cuh).
 constexpr int32_t kAlgoBandExact = 210;
 constexpr int32_t kAlgoIndepExact = 310;
 // Grouped bands: X phase pairs and groups of Z period copies (areas one to a few periods wide).
 constexpr int32_t kAlgoGrouped = 220;
-constexpr int32_t kAlgoGroupedExact = 230;  // grouped bands with bit-sliced exact counts
+constexpr int32_t kAlgoGroupedExact = 230;  // grouped bands as bit planes
 // Grouped bands hold at most this many bands; the rule uses them up to this width in periods.
 constexpr int64_t kGroupedMaxBands = 16;
 constexpr int64_t kGroupedMaxPeriods = 16;
-constexpr int64_t kGroupedExactMinWidth = 9LL << 15;  // exact counts: grouped bands from 2.25 periods
+constexpr int64_t kGroupedExactMinWidth = 9LL << 15;  // bit planes: grouped bands from 2.25 periods
 
 // Band mode (band_geometry) of a band algorithm.
 inline int band_mode_of(int32_t algo) {
@@ -144,7 +144,7 @@ struct Context {
     DeviceBuffer<int64_t> bt_prefix;
     bool band_ready = false;
     // 0 auto, 1 general scan, 2 band engine, 3 independent bands, 4 / 5 the band / independent-band
-    // engine with bit-sliced exact counts, 6 / 7 grouped bands (bounded / exact counts).
+    // engine with bit-sliced exact counts, 6 / 7 grouped bands (bounded / bit planes).
     int32_t engine_override = 0;
     // Engine rule (engine_for; slime_b200_set_engine_rule): the shared-LCG band engine for areas
     // at least band_min_periods periods wide from band_min_threshold, or band_fast_periods wide
@@ -215,7 +215,7 @@ struct Context {
                          ExtChunkResult* results);
     // Sites examined and excluded by the biome filter in the last search.
     int64_t last_biome_examined = 0, last_biome_excluded = 0;
-    // Many searches: those the independent-band kernel can take share one persistent launch.
+    // Many searches: those the band kernels can take share persistent launches, one a class.
     int32_t search_batch(const SearchSpec* q, int32_t n, ExtChunkResult* results, int64_t* totals);
     // Sites and histogram of a finished band search from its emitted hits (already filtered
     // against its rare chunks on the device) plus the rare-chunk fix-up.

@@ -36,7 +36,7 @@ struct Job {
     SearchSpec q{};
     int32_t state = kQueued;
     bool band = false;        // runs in the batch kernel (else: the single search, whole)
-    bool exact = false;       // band work with bit-sliced exact counts
+    bool exact = false;       // band work on bit planes
     bool started = false;
     Clock::time_point t_submit, t_done;
     int64_t total = -1;

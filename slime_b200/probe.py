@@ -8,14 +8,13 @@ library reports them. Cases (sizes chosen so that one launch holds a few GB at m
 under a second):
 
   general40   general_scan_kernel: the 4,001^2 threshold-40 search about (0, 0)
-  exact40     band_scan_kernel, independent bands with bit-sliced exact counts: radius 100,000,
-              threshold 40
+  exact40     plane_kernel, independent bands: radius 100,000, threshold 40
   band60      band_scan_kernel, shared LCG: radius 600,000 (9+ periods), threshold 60
   grouped60   band_scan_kernel, grouped bands: radius 200,000 (3 periods: 4 groups x 4 copies),
               threshold 60
   world60     band_scan_kernel, shared LCG: the full-world threshold-60 scan (36 launches of ~60 ms,
               under 1 GB on the device); profile one launch of it (`-c 1`)
-  precise     precise_kernel: precise AFK scores of the best 20,000 sites of a threshold-36 search
+  precise     precise_one_kernel: precise AFK scores of the best 20,000 sites of a threshold-36 search
   biome       biome chunk_kernel: the Deep Dark / Mushroom Fields filter of 4,096 threshold-48
               sites (version 26.2)
 """
