@@ -10,6 +10,7 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
+#include <new>
 #include <string>
 #include <thread>
 #include <vector>
@@ -175,13 +176,22 @@ void rank_best(std::vector<Hit>& v, const std::vector<uint32_t>& h, const Search
     v.erase(std::remove_if(v.begin(), v.end(), [gate](const Hit& hit) { return hit.count < gate; }), v.end());
     const int64_t x0 = (int64_t)q.center_x - q.rd_max, z0 = (int64_t)q.center_z - q.rd_max, w = 2 * q.rd_max + 1;
     constexpr int64_t kEdge = 1LL << 27;
-    if (n < 64 || x0 < -kEdge || z0 < -kEdge || x0 + w > kEdge || z0 + w > kEdge) {
+    std::vector<uint64_t> key, other;
+    bool packed = n >= 64 && x0 >= -kEdge && z0 >= -kEdge && x0 + w <= kEdge && z0 + w <= kEdge;
+    if (packed) {
+        try {
+            key.resize(n);
+            other.resize(n);
+        } catch (const std::bad_alloc&) {  // no room beside the hits: sort them in place
+            packed = false;
+        }
+    }
+    if (!packed) {
         std::sort(v.begin(), v.end(), hit_better);
         return;
     }
     int bits = 1;
     while ((1LL << bits) < w) ++bits;
-    std::vector<uint64_t> key(n), other(n);
     for (size_t i = 0; i < n; ++i)
         key[i] = ((uint64_t)(221 - v[i].count) << (2 * bits)) | ((uint64_t)(v[i].cx - x0) << bits) | (uint64_t)(v[i].cz - z0);
     constexpr int kDigit = 11;
