@@ -418,7 +418,10 @@ bool Context::scan_band(const SearchSpec& q, std::vector<Hit>& best, std::vector
             if (c >= emit_min) have += h[c];
         }
         const uint64_t need = std::min<uint64_t>(total, (uint64_t)q.max_results);
-        if (have >= need || emit_min <= q.min_size) return true;
+        if (have >= need || emit_min <= q.min_size) {
+            drop_below_gate(best, emit_min);
+            return true;
+        }
         // Too few sites sent: the exact gate (highest count whose cumulative number covers need).
         uint64_t acc = 0;
         int32_t gate = q.max_size;

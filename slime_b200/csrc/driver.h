@@ -1,6 +1,7 @@
 // driver.h -- process-wide state of the C-ABI library (one device, one stream, cached buffers).
 #pragma once
 
+#include <algorithm>
 #include <atomic>
 #include <cstdint>
 #include <mutex>
@@ -105,6 +106,13 @@ inline bool hit_order(const Hit& a, const Hit& b) {
     const int32_t ax = block_of(a.cx), bx = block_of(b.cx);
     if (ax != bx) return ax < bx;
     return block_of(a.cz) < block_of(b.cz);
+}
+
+// A band scan's sites from the emission gate on are complete; of those below it only the ones whose
+// window holds a rare chunk are there (the fix-up lists them whatever their count). They must not rank: a
+// biome exclusion that uses up the others would take them before sites that were not sent.
+inline void drop_below_gate(std::vector<Hit>& sites, int32_t gate) {
+    sites.erase(std::remove_if(sites.begin(), sites.end(), [gate](const Hit& s) { return s.count < gate; }), sites.end());
 }
 
 bool validate_search(int64_t rd_max, int32_t min_size, int32_t max_size, int64_t rd_min,

@@ -284,6 +284,7 @@ int Server::finish_band(Job* j) {
         }
         return 2;
     }
+    drop_below_gate(best, j->emit_min);
     int64_t t = c.finish(j->q, best, h, j->results.data());
     if (t == kNeedMoreSites) t = c.search(j->q, j->results.data());  // biome exclusion needs more sites
     if (t < 0) return 0;
