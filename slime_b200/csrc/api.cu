@@ -164,7 +164,7 @@ void keep_best(std::vector<Hit>& v, size_t k) {
 // comparing records took 200.
 void rank_best(std::vector<Hit>& v, const std::vector<uint32_t>& h, const SearchSpec& q, size_t k) {
     k = std::min(k, v.size());
-    int gate = std::min(q.max_size, 221);
+    int gate = q.max_size;
     for (uint64_t acc = 0; gate > q.min_size; --gate)
         if ((acc += h[gate]) >= k) break;
     const size_t n = (size_t)std::count_if(v.begin(), v.end(), [gate](const Hit& hit) { return hit.count >= gate; });
@@ -499,7 +499,7 @@ int64_t search_entry(int64_t seed, int64_t rd_max, int32_t min_size, int32_t max
                      int32_t cx, int32_t cz, ExtChunkResult* results, int32_t max_results,
                      int32_t precise_afk, int32_t biome_flags = 0, int32_t biome_version = 0) {
     std::lock_guard<std::mutex> lock(ctx().mu);
-    slime::SearchSpec q{seed, rd_max, min_size, max_size, rd_min, cx, cz, max_results, precise_afk,
+    slime::SearchSpec q{seed, rd_max, min_size, slime::upper_bound(max_size), rd_min, cx, cz, max_results, precise_afk,
                         biome_flags, biome_version};
     return ctx().search(q, reinterpret_cast<slime::ExtChunkResult*>(results));
 }
@@ -729,8 +729,8 @@ int32_t slime_b200_search_batch(const SlimeBatchRequest* requests, int32_t n, Ex
     std::vector<slime::SearchSpec> q((size_t)n);
     for (int32_t i = 0; i < n; ++i) {
         const SlimeBatchRequest& r = requests[i];
-        q[i] = slime::SearchSpec{r.seed, r.rd_max, r.min_size, r.max_size, r.rd_min, r.center_x, r.center_z,
-                                 r.max_results, r.precise_afk, r.biome_flags, r.biome_version};
+        q[i] = slime::SearchSpec{r.seed, r.rd_max, r.min_size, slime::upper_bound(r.max_size), r.rd_min, r.center_x,
+                                 r.center_z, r.max_results, r.precise_afk, r.biome_flags, r.biome_version};
     }
     return ctx().search_batch(q.data(), n, reinterpret_cast<slime::ExtChunkResult*>(results), totals);
 }

@@ -38,7 +38,7 @@ int32_t emission_gate(const SearchSpec& q, int64_t ranked) {
     const double centres = w * w - 3.14159265358979 * r * r;
     const double above = tail_share(q.max_size + 1);
     int32_t gate = q.min_size;
-    while (gate < std::min(q.max_size, 221) &&
+    while (gate < q.max_size &&
            centres * (tail_share(gate + 1) - above) >= 4.0 * (double)ranked + 512.0)
         ++gate;
     return gate;

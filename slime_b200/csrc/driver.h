@@ -42,7 +42,7 @@ struct SearchSpec {
     int64_t seed;
     int64_t rd_max;
     int32_t min_size;
-    int32_t max_size;
+    int32_t max_size;  // at most 221 (upper_bound)
     int64_t rd_min;
     int32_t center_x;
     int32_t center_z;
@@ -114,6 +114,9 @@ inline bool hit_order(const Hit& a, const Hit& b) {
 inline void drop_below_gate(std::vector<Hit>& sites, int32_t gate) {
     sites.erase(std::remove_if(sites.begin(), sites.end(), [gate](const Hit& s) { return s.count < gate; }), sites.end());
 }
+
+// A window holds at most 221 cells; callers may give any larger upper bound.
+inline int32_t upper_bound(int32_t max_size) { return std::min(max_size, kHistBins - 1); }
 
 bool validate_search(int64_t rd_max, int32_t min_size, int32_t max_size, int64_t rd_min,
                      int32_t cx, int32_t cz, const void* results, int32_t max_results);

@@ -84,6 +84,7 @@ int64_t search_noalloc(int64_t seed, int64_t rd_max, int32_t min_size, int32_t m
                        int32_t max_results) {
     std::lock_guard<std::mutex> lock(ctx().mu);
     if (!validate_search(rd_max, min_size, max_size, rd_min, cx, cz, results, max_results)) return -1;
+    max_size = upper_bound(max_size);
     if (rd_max > kMaxRadius || max_results > kMaxResults) {
         ctx().set_error_text("no-alloc search: radius above 8191 chunks or max_results above 65536 "
                              "(the fixed 4 MiB scratch array does not hold larger searches)");

@@ -464,8 +464,8 @@ int64_t slime_b200_server_submit(void* server, const SlimeBatchRequest* r) {
     auto* s = static_cast<Server*>(server);
     if (!s || !r) return -1;
     auto j = std::make_unique<slime::Job>();
-    j->q = slime::SearchSpec{r->seed, r->rd_max, r->min_size, r->max_size, r->rd_min, r->center_x, r->center_z,
-                             r->max_results, r->precise_afk, r->biome_flags, r->biome_version};
+    j->q = slime::SearchSpec{r->seed, r->rd_max, r->min_size, slime::upper_bound(r->max_size), r->rd_min, r->center_x,
+                             r->center_z, r->max_results, r->precise_afk, r->biome_flags, r->biome_version};
     std::vector<ExtChunkResult> probe(1);
     if (!slime::validate_search(j->q.rd_max, j->q.min_size, j->q.max_size, j->q.rd_min, j->q.center_x,
                                 j->q.center_z, reinterpret_cast<slime::ExtChunkResult*>(probe.data()),
