@@ -162,7 +162,7 @@ void keep_best(std::vector<Hit>& v, size_t k) {
 // chunks (block coordinates do not wrap) a hit packs into one word whose order is the ranking, and the
 // words are radix-sorted 11 bits at a time: 2,629 sites of a radius-2,000 search take about 20 us where
 // comparing records took 200.
-void rank_best(std::vector<Hit>& v, const std::vector<uint32_t>& h, const SearchSpec& q, size_t k) {
+void rank_best(std::vector<Hit>& v, const Counts& h, const SearchSpec& q, size_t k) {
     k = std::min(k, v.size());
     int gate = q.max_size;
     for (uint64_t acc = 0; gate > q.min_size; --gate)
@@ -228,7 +228,7 @@ bool validate_search(int64_t rd_max, int32_t min_size, int32_t max_size, int64_t
 }
 
 // Scans one area with the general engine; fills `best` (<= max_results, unsorted) and `hist`.
-bool Context::scan_general(const SearchSpec& q, std::vector<Hit>& best, std::vector<uint32_t>& h,
+bool Context::scan_general(const SearchSpec& q, std::vector<Hit>& best, Counts& h,
                            bool& cancelled) {
     const int64_t width = 2 * q.rd_max + 1;
     const int32_t area_x0 = (int32_t)((int64_t)q.center_x - q.rd_max);
@@ -241,7 +241,10 @@ bool Context::scan_general(const SearchSpec& q, std::vector<Hit>& best, std::vec
     const int out_w = general_out_width();
     const int tiles_x = (int)((width + out_w - 1) / out_w);
     const int64_t height = width;
-    const int band_h = general_band_rows(width, height, sm_count);
+    // A launch's counts go to 32-bit bins, the fullest of which takes 9.3 % of its centres.
+    constexpr double kMostCentres = 4.5e10;
+    int band_h = general_band_rows(width, height, sm_count);
+    while (band_h > 8 && (double)width * band_h > kMostCentres) band_h -= 8;
     const uint64_t cap = hits.count - kScanHeader;
     Hit* const first_hits = reinterpret_cast<Hit*>((char*)pinned + kScanHeaderBytes);
     // Counts below the gate are only histogrammed; the exact histogram decides afterwards whether a
@@ -256,6 +259,7 @@ bool Context::scan_general(const SearchSpec& q, std::vector<Hit>& best, std::vec
         int64_t slab = std::min<int64_t>(height, std::max<int64_t>(band_h, (int64_t)(4e10 / width)));
         if (per_row > 0) slab = std::min<int64_t>(slab, std::max<int64_t>(band_h, (int64_t)(cap / 4 / per_row)));
         slab = (slab + band_h - 1) / band_h * band_h;  // whole patches: an area that fits runs in one launch
+        slab = std::min<int64_t>(slab, std::max<int64_t>(band_h, (int64_t)(kMostCentres / width) / band_h * band_h));
         for (int64_t z0 = 0; z0 < height;) {
             while (paused.load() && !cancel.load()) std::this_thread::sleep_for(std::chrono::milliseconds(20));
             if (cancel.load()) { cancelled = true; return true; }
@@ -385,7 +389,7 @@ int64_t Context::search(const SearchSpec& q, ExtChunkResult* results) {
     last_launches = 0;
     last_biome_examined = last_biome_excluded = 0;
     std::vector<Hit> best;
-    std::vector<uint32_t> h(kHistBins, 0u);
+    Counts h(kHistBins, 0);
     bool cancelled = false;
     last_rare = 0;
     const int32_t algo = engine_for(q);
@@ -420,7 +424,7 @@ int64_t Context::search(const SearchSpec& q, ExtChunkResult* results) {
 
 // Biome exclusion after a scan: the ranked sites are filtered in rank order, a few thousand at a
 // time, until max_results pass (verdict mask & flags == 0) or the sites run out.
-int64_t Context::finish_biome(const SearchSpec& q, std::vector<Hit>& best, const std::vector<uint32_t>& h, int64_t total,
+int64_t Context::finish_biome(const SearchSpec& q, std::vector<Hit>& best, const Counts& h, int64_t total,
                               ExtChunkResult* results) {
     rank_best(best, h, q, best.size());
     const int32_t flags = q.biome_flags & 3, large = (q.biome_flags >> 2) & 1;
@@ -466,7 +470,7 @@ int64_t Context::finish_biome(const SearchSpec& q, std::vector<Hit>& best, const
     return total;
 }
 
-int64_t Context::finish(const SearchSpec& q, std::vector<Hit>& best, const std::vector<uint32_t>& h,
+int64_t Context::finish(const SearchSpec& q, std::vector<Hit>& best, const Counts& h,
                         ExtChunkResult* results) {
     int64_t total = 0;
     for (int s = q.min_size; s <= q.max_size; ++s) total += h[s];

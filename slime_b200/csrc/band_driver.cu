@@ -166,7 +166,7 @@ int band_class(const BandArgs& a) {
     return 4 + 3 * mode + (joined == 4 ? 2 : joined - 1);
 }
 
-bool Context::scan_band(const SearchSpec& q, std::vector<Hit>& best, std::vector<uint32_t>& h,
+bool Context::scan_band(const SearchSpec& q, std::vector<Hit>& best, Counts& h,
                         bool& cancelled, int mode, bool exact) {
     if (!ensure_band()) return false;
     const int64_t W = 2 * q.rd_max + 1, H = W;
@@ -411,7 +411,7 @@ bool Context::scan_band(const SearchSpec& q, std::vector<Hit>& best, std::vector
         }
         const uint32_t* hs = (const uint32_t*)((const char*)pinned + 64);
         const int32_t* hd = (const int32_t*)(hs + kHistBins);
-        for (int i = 0; i < kHistBins; ++i) h[i] = (uint32_t)((int64_t)hs[i] + hd[i]);
+        for (int i = 0; i < kHistBins; ++i) h[i] = (uint64_t)((int64_t)hs[i] + hd[i]);
         uint64_t total = 0, have = 0;
         for (int c = q.min_size; c <= q.max_size; ++c) {
             total += h[c];

@@ -97,7 +97,7 @@ cudaError_t run_band_items(std::vector<BandArgs>& items, BandArgs* args_dev, int
 
 bool Context::collect_band(const SearchSpec& q, int32_t area_x0, int32_t area_z0, const Hit* hits_host,
                            uint64_t n, const int2* rare_dev, uint32_t nrare, unsigned long long* fixed_count_dev,
-                           unsigned int* ferr_dev, std::vector<Hit>& best, std::vector<uint32_t>& h) {
+                           unsigned int* ferr_dev, std::vector<Hit>& best, Counts& h) {
     std::fill(h.begin(), h.end(), 0u);
     best.clear();
     best.reserve(n);
@@ -338,7 +338,7 @@ int32_t Context::search_batch(const SearchSpec* reqs, int32_t n, ExtChunkResult*
     }
 
     // ---- per search: fix-up, histogram, ranking, precise scores ------------------------------
-    std::vector<uint32_t> h(kHistBins, 0u);
+    Counts h(kHistBins, 0);
     for (int32_t s = 0; s < m; ++s) {
         const Planned& p = plan[s];
         const SearchSpec& q = reqs[p.idx];

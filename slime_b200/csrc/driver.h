@@ -53,6 +53,9 @@ struct SearchSpec {
     int32_t biome_version = 0;  // Minecraft version code of the biome tree (e.g. 2602)
 };
 
+// Centres in range by count, of a whole search (a full-world search holds 1.4e13).
+using Counts = std::vector<uint64_t>;
+
 constexpr int64_t kNeedMoreSites = -3;  // finish(): the biome exclusion needs more ranked sites
 
 // Values reported by get_gpu_v1_algorithm().
@@ -209,20 +212,20 @@ struct Context {
     void release();
     void release_extra();
 
-    bool scan_general(const SearchSpec& q, std::vector<Hit>& best, std::vector<uint32_t>& hist_out,
+    bool scan_general(const SearchSpec& q, std::vector<Hit>& best, Counts& hist_out,
                       bool& cancelled);
     bool ensure_band();
     int32_t engine_for(const SearchSpec& q) const;
-    bool scan_band(const SearchSpec& q, std::vector<Hit>& best, std::vector<uint32_t>& hist_out,
+    bool scan_band(const SearchSpec& q, std::vector<Hit>& best, Counts& hist_out,
                    bool& cancelled, int mode, bool exact = false);
     bool score(int64_t seed, ExtChunkResult* host, int32_t n, int32_t scan_xz, bool pack);
     int64_t search(const SearchSpec& q, ExtChunkResult* results);
     // Total in range, ranked results and precise scores of a finished scan (-1 on failure). With
     // a biome exclusion the results are the best sites whose window passes the filter; when
     // fewer than max_results pass and `best` misses sites of the area, kNeedMoreSites.
-    int64_t finish(const SearchSpec& q, std::vector<Hit>& best, const std::vector<uint32_t>& h,
+    int64_t finish(const SearchSpec& q, std::vector<Hit>& best, const Counts& h,
                    ExtChunkResult* results);
-    int64_t finish_biome(const SearchSpec& q, std::vector<Hit>& best, const std::vector<uint32_t>& h, int64_t total,
+    int64_t finish_biome(const SearchSpec& q, std::vector<Hit>& best, const Counts& h, int64_t total,
                          ExtChunkResult* results);
     // Sites examined and excluded by the biome filter in the last search.
     int64_t last_biome_examined = 0, last_biome_excluded = 0;
@@ -232,7 +235,7 @@ struct Context {
     // against its rare chunks on the device) plus the rare-chunk fix-up.
     bool collect_band(const SearchSpec& q, int32_t area_x0, int32_t area_z0, const Hit* hits_host, uint64_t n,
                       const int2* rare_dev, uint32_t nrare, unsigned long long* fixed_count_dev,
-                      unsigned int* ferr_dev, std::vector<Hit>& best, std::vector<uint32_t>& h);
+                      unsigned int* ferr_dev, std::vector<Hit>& best, Counts& h);
 };
 
 Context& ctx();

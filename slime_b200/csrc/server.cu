@@ -255,8 +255,8 @@ int Server::finish_band(Job* j) {
         c.set_error("server histogram", e);
         return 0;
     }
-    std::vector<uint32_t> h(kHistBins, 0u);
-    for (int i = 0; i < kHistBins; ++i) h[i] = (uint32_t)((int64_t)hd[i] + (int32_t)hd[kHistBins + i]);
+    Counts h(kHistBins, 0);
+    for (int i = 0; i < kHistBins; ++i) h[i] = (uint64_t)((int64_t)hd[i] + (int32_t)hd[kHistBins + i]);
     uint64_t total = 0, have = 0;
     for (int k = j->q.min_size; k <= j->q.max_size; ++k) {
         total += h[k];
