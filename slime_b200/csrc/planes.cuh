@@ -95,6 +95,10 @@ struct __align__(16) PlaneSmem {
     uint32_t list[kListCap];                  // unions waiting for their windows' counts
     unsigned int listed;
     unsigned int hist[kHistBins];             // counts of this CTA's centres in range (if args.hist)
+    // Of the current tile's search, by band: first area row (before the tile's base row), and with grouped
+    // bands the base row from which its rows belong to the next copy's first group.
+    int64_t row0[kMaxBands];
+    int32_t row_end[kGrpBands];
 };
 static_assert(sizeof(PlaneSmem) <= (233472 - 2048) / kCtasPerSm, "two CTAs an SM");
 
@@ -134,14 +138,6 @@ struct Tile {
     uint32_t mask;  // their bits in a row's valid mask
     int groups, min_size, max_size;
 };
-
-// First area row (band axis) of band m, before the tile's base row is added.
-template <int kMode>
-__device__ __forceinline__ int64_t band_row0(const BandArgs& a, int m) {
-    if (kMode != kModeGrouped) return (int64_t)(a.j0 + m) * a.row_stride;
-    const int copies = a.nb / a.groups;
-    return (int64_t)(m % copies) * kPeriod + (int64_t)(m / copies) * a.row_stride;
-}
 
 // ---- bit-sliced adders: bit j of every word belongs to combo j ----------------------------------
 
@@ -392,9 +388,8 @@ __device__ __forceinline__ void keep_centre(PlaneSmem& S, const BandArgs& a, con
     if (m >= a.nb || c < 0 || c >= Shape<kMode>::kOutW || rr < 0 || rr >= T.out_h) return;
     const int64_t u = (int64_t)T.u0 + c;
     const int64_t cu = u + (int64_t)(T.i0 + ph) * kPeriod;
-    const int64_t cv = (int64_t)T.v0 + rr + band_row0<kMode>(a, m);
-    // Grouped bands: rows of the last group past the period belong to the next copy's first group.
-    if (kMode == kModeGrouped && T.copies > 1 && T.v0 + rr + (m / T.copies) * a.row_stride >= kPeriod) return;
+    const int64_t cv = (int64_t)T.v0 + rr + S.row0[m];
+    if (kMode == kModeGrouped && T.v0 + rr >= S.row_end[m]) return;
     if (u >= a.ubase || cu >= a.width_u || cv >= a.height_v) return;
     const int32_t cx = (int32_t)(a.transposed ? a.area_x0 + cv : a.area_x0 + cu);
     const int32_t cz = (int32_t)(a.transposed ? a.area_z0 + cu : a.area_z0 + cv);
@@ -700,6 +695,14 @@ __device__ __forceinline__ bool plane_tile(PlaneSmem& S, const BandArgs& a, int6
 #pragma unroll
         for (int i = 0; i < Counter<kUnion>::kP; ++i) E.cnt[u][i] = 0;
     for (int i = tid; i < kRingWords / 4; i += kTpb) reinterpret_cast<uint4*>(S.ring)[i] = make_uint4(0u, 0u, 0u, 0u);
+    // Worked out a kept centre at a time, the bands' rows cost five divisions each: grouped bands at thresholds
+    // below 40 took up to twice as long (radius 180,000, threshold 37: 252 ms).
+    if (tid < kMaxBands) {
+        const int copy = tid % T.copies, group = tid / T.copies;
+        S.row0[tid] = kMode == kModeGrouped ? copy * kPeriod + group * a.row_stride : (a.j0 + tid) * a.row_stride;
+        if (kMode == kModeGrouped && tid < kGrpBands)
+            S.row_end[tid] = T.copies > 1 ? (int32_t)max((int64_t)0, kPeriod - group * a.row_stride) : INT32_MAX;
+    }
     // Row terms of batches 0 and 1 (batch b lives in rows[b % 2]).
     if (tid == 0) {
         bulk_load(&S.rows[0][0], a.rt + (int64_t)T.v0 * kRW, kBatchBytes, &S.rows_bar[0]);
