@@ -136,8 +136,8 @@ void slime_b200_set_engine(int32_t mode, int32_t band_min_threshold);
  * grouped_max_width, exact_wide_below_threshold}. The shared-LCG band engine takes areas at least
  * band_min_periods x 2^17 chunks wide from band_min_threshold, or band_fast_periods x 2^17 wide from
  * band_fast_threshold; grouped bands (X phase pairs x groups of Z period copies) take areas
- * grouped_min_width .. grouped_max_width chunks wide (at most 16 x 2^17) from grouped_min_threshold,
- * before the shared LCG. Of the others, thresholds below exact_below_threshold (on areas 2.25 x 2^17
+ * grouped_min_width chunks wide and wider (at most 16 x 2^17) from grouped_min_threshold: up to
+ * grouped_max_width before the shared LCG, past it where neither of its branches applies. Of the others, thresholds below exact_below_threshold (on areas 2.25 x 2^17
  * chunks wide or more: below exact_wide_below_threshold) on areas of exact_min_centres centres or more
  * use the bit-plane kernels with exact counts (independent bands; from 2.25 x 2^17 grouped bands; from
  * 16 x 2^17 the shared LCG) while the expected number of sites stays below 1e9. Independent bands take
@@ -150,6 +150,9 @@ void slime_b200_set_engine(int32_t mode, int32_t band_min_threshold);
  * B200 measurements. */
 int32_t slime_b200_set_engine_rule(const int64_t* rule, int32_t n);
 int32_t slime_b200_get_engine_rule(int64_t* rule, int32_t n);
+/* The engine (as get_gpu_v1_algorithm() reports it) that the current mode and rule choose for a search of
+ * this radius, threshold and inner radius; -1 for arguments out of range. Needs no device. */
+int32_t slime_b200_engine_for(int64_t rd_max, int32_t min_size, int64_t rd_min);
 
 /* Generator variant of earlier versions; accepted and without effect (results never depended on it). */
 void slime_b200_set_tuning(int32_t band_mad_add);

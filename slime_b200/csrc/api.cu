@@ -726,6 +726,13 @@ int32_t slime_b200_get_engine_rule(int64_t* rule, int32_t n) {
     return 0;
 }
 
+int32_t slime_b200_engine_for(int64_t rd_max, int32_t min_size, int64_t rd_min) {
+    if (rd_max < 0 || rd_max > (INT32_MAX - 19LL) / 2LL || min_size < 0 || min_size > 221 || rd_min < 0 || rd_min > rd_max)
+        return -1;
+    std::lock_guard<std::mutex> lock(ctx().mu);
+    return ctx().engine_for(slime::SearchSpec{0, rd_max, min_size, slime::kHistBins - 1, rd_min, 0, 0, 1, 0});
+}
+
 int32_t slime_b200_search_batch(const SlimeBatchRequest* requests, int32_t n, ExtChunkResult* results,
                                 int64_t* totals) {
     std::lock_guard<std::mutex> lock(ctx().mu);

@@ -176,8 +176,8 @@ struct Context {
     // bit-plane kernels with exact counts, as long as the expected number of sites stays below 1e9.
     int32_t exact_below_threshold = 55;
     int64_t exact_min_centres = 400040001;
-    // Grouped bands for areas grouped_min_width .. grouped_max_width chunks wide (at most
-    // kGroupedMaxPeriods periods) from grouped_min_threshold.
+    // Grouped bands for areas of grouped_min_width chunks and more (at most kGroupedMaxPeriods periods) from
+    // grouped_min_threshold; past grouped_max_width only where the shared LCG's branches do not apply.
     int32_t grouped_min_threshold = 55;
     int32_t exact_wide_below_threshold = 55;
     int64_t grouped_min_width = 200001;

@@ -60,6 +60,7 @@ SIGNATURES = {
     "slime_b200_search_batch": (i32, [vp, i32, vp, vp]),
     "slime_b200_set_engine_rule": (i32, [vp, i32]),
     "slime_b200_get_engine_rule": (i32, [vp, i32]),
+    "slime_b200_engine_for": (i32, [i64, i32, i64]),
     "slime_b200_server_create": (vp, [i64, i32]),
     "slime_b200_server_submit": (i64, [vp, vp]),
     "slime_b200_server_poll": (i32, [vp, i64]),

@@ -1,0 +1,49 @@
+"""The engine rule over widths and thresholds (no device needed): what the library picks where the branches
+of the rule meet."""
+import pytest
+
+PERIOD = 1 << 17
+GENERAL, SHARED, GROUPED, INDEPENDENT = 100, 200, 220, 300
+
+
+@pytest.fixture(scope="module")
+def core():
+    from slime_b200 import build
+    from slime_b200.lib import SlimeCoreB200
+    build.build()
+    core = SlimeCoreB200()
+    core.lib.slime_b200_set_engine(0, 0)
+    return core
+
+
+def test_wide_areas_always_share_the_generator(core):
+    """Areas several periods wide cost independent bands about twice the time of the modes that share work
+    between periods: at no width and threshold may the branches leave a gap that sends them there."""
+    radii = {int(147_456 * 1.02**i) for i in range(129)}
+    for n in range(3, 29):  # on both sides of every period
+        radii |= {(n * PERIOD - 1) // 2 + d for d in (-1, 0, 1)}
+    radii |= {100_000 * k + d for k in range(2, 19) for d in (-1, 0, 1)} | {1_875_000}
+    for r in sorted(r for r in radii if 147_456 <= r <= 1_875_000):
+        for threshold in range(42, 90):
+            assert core.lib.slime_b200_engine_for(r, threshold, 0) not in (GENERAL, INDEPENDENT), (r, threshold)
+
+
+def test_grouped_bands_go_on_to_the_shared_lcg(core):
+    for threshold in (55, 60, 75):
+        for r in (500_000, 500_001, 510_000, 524_287):
+            assert core.lib.slime_b200_engine_for(r, threshold, 0) == GROUPED
+        assert core.lib.slime_b200_engine_for(524_288, threshold, 0) == SHARED
+
+
+def test_a_disabled_branch_stays_off(core):
+    before = core.engine_rule()
+    try:
+        core.set_engine_rule(dict(before, grouped_min_threshold=222))
+        assert core.lib.slime_b200_engine_for(510_000, 60, 0) == INDEPENDENT
+    finally:
+        core.set_engine_rule(before)
+
+
+def test_arguments_out_of_range(core):
+    for args in ((-1, 40, 0), (10, 222, 0), (10, -1, 0), (10, 40, 11), (10, 40, -1), (2**31, 40, 0)):
+        assert core.lib.slime_b200_engine_for(*args) == -1
