@@ -66,11 +66,22 @@ int32_t Context::engine_for(const SearchSpec& q) const {
     // 4.6 / 15.3 periods; the shared LCG 1.54 / 2.43 / 2.86 at 9.2 / 15.3 / 19.1.
     constexpr double kExactMaxSites = 1e9;
     if (!shared && !grouped && q.min_size < (wide ? exact_wide_below_threshold : exact_below_threshold) &&
-        w * w >= exact_min_centres && (double)w * (double)w * tail_share(q.min_size) <= kExactMaxSites)
-        // Independent bands run the same kernels either way; counted by unions of windows they are
-        // reported as bounded.
-        return !wide ? (plane_union(q.min_size) > 1 ? kAlgoIndep : kAlgoIndepExact)
-               : copies_fit ? kAlgoGroupedExact : kAlgoBandExact;
+        w * w >= exact_min_centres && (double)w * (double)w * tail_share(q.min_size) <= kExactMaxSites) {
+        const bool single = plane_union(q.min_size) == 1;  // every window counted by itself: thresholds below 40
+        // Bit planes count all combos of a column at once, those inside the rd_min disc too; the general scan
+        // skips the patches there. From these shares of the area outside the disc on down it is the faster one
+        // on wide areas at low thresholds. B200, inner radius 0.8 / 0.9 / 0.99 of the outer: radius 400,000,
+        // threshold 39 480 / 357 / 234 ms against 495 / 490 / 486; 900,000 at 40 2,382 / 1,772 / 1,161 against
+        // 1,694 / 1,692 / 1,690. Narrower areas and thresholds from 41 on lose nothing to the disc.
+        const double outside = 1.0 - 3.14159265358979 * (double)q.rd_min * (double)q.rd_min / ((double)w * (double)w);
+        if (wide && outside < (single ? 0.5 : q.min_size == 40 ? 0.36 : 0.0)) return kAlgoGeneral;
+        // Single windows cost more to count than to generate, and grouped bands leave bits of a word empty:
+        // they start at 4 periods there (radius 200,000, threshold 39 160 ms against 129 with independent
+        // bands; 262,144: 218 against 221). Independent bands run the same kernels either way; counted by
+        // unions of windows they are reported as bounded.
+        if (!wide || (single && w < kGroupedSingleMinWidth)) return single ? kAlgoIndepExact : kAlgoIndep;
+        return copies_fit ? kAlgoGroupedExact : kAlgoBandExact;
+    }
     if (grouped) return kAlgoGrouped;
     if (shared) return kAlgoBand;
     if (w * w >= indep_min_centres && q.min_size >= indep_min_threshold) return kAlgoIndep;

@@ -72,6 +72,7 @@ constexpr int32_t kAlgoGroupedExact = 230;  // grouped bands as bit planes
 constexpr int64_t kGroupedMaxBands = 16;
 constexpr int64_t kGroupedMaxPeriods = 16;
 constexpr int64_t kGroupedExactMinWidth = 9LL << 15;  // bit planes: grouped bands from 2.25 periods
+constexpr int64_t kGroupedSingleMinWidth = 4LL << 17;  // where each window is counted by itself: from 4
 
 // Band mode (band_geometry) of a band algorithm.
 inline int band_mode_of(int32_t algo) {

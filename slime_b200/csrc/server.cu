@@ -97,7 +97,10 @@ namespace {
 void plan_job(Job& j, const Context& c) {
     const SearchSpec& q = j.q;
     const int64_t W = 2 * q.rd_max + 1;
-    const int32_t algo = c.engine_for(q);
+    // Whatever the inner radius: a general scan would hold every other request for its whole length.
+    SearchSpec full = q;
+    full.rd_min = 0;
+    const int32_t algo = c.engine_for(full);
     const double centres = (double)W * (double)W;
     // Emission gate, as the single search chooses it (biome requests keep more, as there).
     const int64_t want = (q.biome_flags & 3) ? 2LL * q.max_results + 1024 : (int64_t)q.max_results;

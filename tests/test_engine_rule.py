@@ -47,3 +47,22 @@ def test_a_disabled_branch_stays_off(core):
 def test_arguments_out_of_range(core):
     for args in ((-1, 40, 0), (10, 222, 0), (10, -1, 0), (10, 40, 11), (10, 40, -1), (2**31, 40, 0)):
         assert core.lib.slime_b200_engine_for(*args) == -1
+
+
+def test_thin_annuli_of_low_thresholds_take_the_general_scan(core):
+    pick = core.lib.slime_b200_engine_for
+    for r, threshold in ((147_456, 36), (200_000, 39), (400_000, 37), (690_000, 39), (150_000, 40), (900_000, 40)):
+        inside, outside = (0.75, 0.85) if threshold < 40 else (0.85, 0.95)
+        assert pick(r, threshold, int(outside * r)) == GENERAL
+        assert pick(r, threshold, int(inside * r)) == pick(r, threshold, 0) != GENERAL
+    for r in (147_456, 400_000, 900_000):
+        for threshold in (41, 42, 50, 60):
+            assert pick(r, threshold, r) == pick(r, threshold, 0) != GENERAL
+    assert pick(100_000, 39, 99_000) == pick(100_000, 39, 0) != GENERAL  # narrow areas stay
+
+
+def test_single_windows_of_narrow_areas_take_independent_bands(core):
+    pick = core.lib.slime_b200_engine_for
+    for r in (147_456, 200_000, 262_143):
+        assert pick(r, 39, 0) == 310 and pick(r, 40, 0) == 230
+    assert pick(262_144, 39, 0) == 230
