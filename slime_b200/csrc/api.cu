@@ -167,7 +167,7 @@ void rank_best(std::vector<Hit>& v, const Counts& h, const SearchSpec& q, size_t
     int gate = q.max_size;
     for (uint64_t acc = 0; gate > q.min_size; --gate)
         if ((acc += h[gate]) >= k) break;
-    const size_t n = (size_t)std::count_if(v.begin(), v.end(), [gate](const Hit& hit) { return hit.count >= gate; });
+    size_t n = (size_t)std::count_if(v.begin(), v.end(), [gate](const Hit& hit) { return hit.count >= gate; });
     if (n < k) {  // not the histogram of these hits
         if (v.size() > k) std::nth_element(v.begin(), v.begin() + (ptrdiff_t)k, v.end(), hit_better);
         std::sort(v.begin(), v.begin() + (ptrdiff_t)k, hit_better);
@@ -176,24 +176,34 @@ void rank_best(std::vector<Hit>& v, const Counts& h, const SearchSpec& q, size_t
     v.erase(std::remove_if(v.begin(), v.end(), [gate](const Hit& hit) { return hit.count < gate; }), v.end());
     const int64_t x0 = (int64_t)q.center_x - q.rd_max, z0 = (int64_t)q.center_z - q.rd_max, w = 2 * q.rd_max + 1;
     constexpr int64_t kEdge = 1LL << 27;
+    const bool packed = n >= 64 && x0 >= -kEdge && z0 >= -kEdge && x0 + w <= kEdge && z0 + w <= kEdge;
+    int bits = 1;
+    while ((1LL << bits) < w) ++bits;
     std::vector<uint64_t> key, other;
-    bool packed = n >= 64 && x0 >= -kEdge && z0 >= -kEdge && x0 + w <= kEdge && z0 + w <= kEdge;
-    if (packed) {
-        try {
-            key.resize(n);
-            other.resize(n);
-        } catch (const std::bad_alloc&) {  // no room beside the hits: sort them in place
-            packed = false;
-        }
+    try {
+        if (packed) key.reserve(n);
+        if (packed) other.reserve(std::min(n, 2 * k));
+    } catch (const std::bad_alloc&) {  // no room beside the hits: rank them in place
     }
-    if (!packed) {
+    if (key.capacity() < n || other.capacity() < std::min(n, 2 * k)) {
+        if (n > k) {
+            std::nth_element(v.begin(), v.begin() + (ptrdiff_t)k, v.end(), hit_better);
+            v.resize(k);
+        }
         std::sort(v.begin(), v.end(), hit_better);
         return;
     }
-    int bits = 1;
-    while ((1LL << bits) < w) ++bits;
-    for (size_t i = 0; i < n; ++i)
-        key[i] = ((uint64_t)(221 - v[i].count) << (2 * bits)) | ((uint64_t)(v[i].cx - x0) << bits) | (uint64_t)(v[i].cz - z0);
+    for (const Hit& hit : v)
+        key.push_back(((uint64_t)(221 - hit.count) << (2 * bits)) | ((uint64_t)(hit.cx - x0) << bits) | (uint64_t)(hit.cz - z0));
+    // Many sites may share the gate's count (an upper bound can stop the emission gate): then those that rank
+    // are picked out first.
+    if (n > 2 * k) {
+        std::nth_element(key.begin(), key.begin() + (ptrdiff_t)k, key.end());
+        n = k;
+        key.resize(n);
+        v.resize(n);
+    }
+    other.resize(n);
     constexpr int kDigit = 11;
     for (int shift = 0; shift < 2 * bits + 8; shift += kDigit) {
         uint32_t at[1 << kDigit] = {};

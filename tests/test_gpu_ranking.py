@@ -1,0 +1,38 @@
+"""Ranking when far more sites share the lowest count that ranks than can be returned: an upper bound stops
+the emission gate there. The best of the threshold's sites must come in order, ties by block x, then z."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def core():
+    from slime_b200.lib import SlimeCoreB200
+    return SlimeCoreB200()
+
+
+# (radius, low, high, mode): 64 and more ties for each ranked site, and few of them
+@pytest.mark.parametrize("radius,low,high,mode", [(700, 30, 31, 5), (700, 30, 31, 7), (1200, 28, 28, 5), (300, 30, 33, 5)])
+@pytest.mark.parametrize("top", [1, 2, 63, 64, 100, 1000, 5000])
+def test_ties_at_the_gate(core, oracle, radius, low, high, mode, top):
+    core.lib.slime_b200_set_engine(mode, 0)
+    try:
+        total, got = core.search(31337, radius, low, high, 0, 4_000, -9_000, top)
+    finally:
+        core.lib.slime_b200_set_engine(0, 0)
+    want_total, want = oracle.search(31337, radius, low, high, 0, 4_000, -9_000, top)
+    assert total == want_total
+    assert np.array_equal(got, want)
+
+
+def test_ties_where_block_coordinates_wrap(core, oracle):
+    """Past 2^27 chunks the order is that of wrapped 32-bit block coordinates."""
+    core.lib.slime_b200_set_engine(5, 0)
+    try:
+        total, got = core.search(99, 400, 30, 31, 0, 2**27, -(2**27), 50)
+    finally:
+        core.lib.slime_b200_set_engine(0, 0)
+    want_total, want = oracle.search(99, 400, 30, 31, 0, 2**27, -(2**27), 50)
+    assert total == want_total
+    assert np.array_equal(got, want)
