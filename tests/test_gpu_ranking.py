@@ -36,3 +36,17 @@ def test_ties_where_block_coordinates_wrap(core, oracle):
     want_total, want = oracle.search(99, 400, 30, 31, 0, 2**27, -(2**27), 50)
     assert total == want_total
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("radius,low,high,mode", [(6000, 26, 27, 5), (6000, 26, 27, 7), (6000, 27, 27, 4)])
+def test_more_sites_at_the_gate_than_the_hit_buffer_holds(core, radius, low, high, mode):
+    """Five million sites share the highest count in range; the general scan is the check."""
+    results = []
+    for m in (1, mode):
+        core.lib.slime_b200_set_engine(m, 0)
+        try:
+            results.append(core.search(-5, radius, low, high, 0, 77_000, 1_000, 20_000))
+        finally:
+            core.lib.slime_b200_set_engine(0, 0)
+    assert results[0][0] == results[1][0]
+    assert np.array_equal(results[0][1], results[1][1])
