@@ -267,7 +267,8 @@ bool Context::scan_general(const SearchSpec& q, std::vector<Hit>& best, Counts& 
         // Rows per launch: ~4e10 centres, and an expected emission of at most cap / 4.
         const double per_row = (double)width * tail_share(emit_min);
         int64_t slab = std::min<int64_t>(height, std::max<int64_t>(band_h, (int64_t)(4e10 / width)));
-        if (per_row > 0) slab = std::min<int64_t>(slab, std::max<int64_t>(band_h, (int64_t)(cap / 4 / per_row)));
+        const double fitting = (double)(cap / 4) / std::max(per_row, 1e-9);  // no sites expected: no limit
+        if (fitting < (double)slab) slab = std::max<int64_t>(band_h, (int64_t)fitting);
         slab = (slab + band_h - 1) / band_h * band_h;  // whole patches: an area that fits runs in one launch
         slab = std::min<int64_t>(slab, std::max<int64_t>(band_h, (int64_t)(kMostCentres / width) / band_h * band_h));
         for (int64_t z0 = 0; z0 < height;) {
