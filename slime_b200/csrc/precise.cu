@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(kPreciseTpb) precise_kernel(const PreciseArgs 
     const int side = a.scan_xz ? 9 : 1;
     const int pairs = side * side * a.y_count;
 
-    for (int site = blockIdx.x; site < a.n; site += gridDim.x) {
+    for (int64_t site = blockIdx.x; site < a.n; site += gridDim.x) {
         const int64_t bx = a.sites[site].center_x, bz = a.sites[site].center_z;
         const int64_t ux0 = floor_div16(bx + lo) - 10, uz0 = floor_div16(bz + lo) - 10;
         const int nx = (int)(floor_div16(bx + hi) + 10 - ux0 + 1);
@@ -168,78 +168,84 @@ __global__ void __launch_bounds__(kOneTpb) precise_one_kernel(const PreciseArgs 
     const int lo = a.scan_xz ? -16 : 0, hi = a.scan_xz ? 16 : 0;
     const int side = a.scan_xz ? 9 : 1, pairs = side * side;
     int loaded = -1;  // alignment class (both centres mod 4) of the table
+    auto class_of = [&](int64_t s) { return (int)(a.sites[s].center_x & 3) * 4 + (int)(a.sites[s].center_z & 3); };
 
-    for (int first = blockIdx.x * chunk; first < a.n; first += gridDim.x * chunk) {
-        const int last = min(first + chunk, a.n);
-        // Sites of one class at a time: the table's slices are its 16 alignments. Search results are all
-        // of class 0 (centres at 8 mod 16).
-        for (int done = 0; done < last - first;) {
-            int cls = 16;  // the smallest class not yet done
-            for (int s = first; s < last; ++s) {
-                const int c = (int)(a.sites[s].center_x & 3) * 4 + (int)(a.sites[s].center_z & 3);
-                if (c < cls && c >= (done ? loaded + 1 : 0)) cls = c;
+    for (int64_t first = (int64_t)blockIdx.x * chunk; first < a.n; first += (int64_t)gridDim.x * chunk) {
+        const int64_t last = min(first + chunk, (int64_t)a.n);
+        // The offsets of a site meet 16 alignments, the same for all sites of a class. Search results are all of
+        // class 0 (centres at 8 mod 16); a chunk of sites of several classes looks its entries up in global
+        // memory. (A table for each class of a chunk in turn: 5,000 sites of random alignment 224 us a call
+        // against 182 with a CTA a site.)
+        const int cls = class_of(first);
+        bool same = true;
+        for (int64_t s = first + 1 + lane; s < last; s += 32) same &= class_of(s) == cls;
+        const bool shared = __all_sync(0xFFFFFFFFu, same);  // the same in every warp
+        if (shared && cls != loaded) {
+            __syncthreads();  // the previous table is no longer read
+            for (int e = tid; e < 16 * kSlice / 8; e += kOneTpb) {
+                const int s = e / (kSlice / 8), ax = (s >> 2) * 4 + (cls >> 2), az = (s & 3) * 4 + (cls & 3);
+                reinterpret_cast<uint4*>(table)[e] =
+                    reinterpret_cast<const uint4*>(a.weights + (ax * 16 + az) * kSlice)[e % (kSlice / 8)];
             }
-            if (cls != loaded || !done) {
-                __syncthreads();  // the previous table is no longer read
-                if (cls != loaded)
-                    for (int e = tid; e < 16 * kSlice / 8; e += kOneTpb) {
-                        const int s = e / (kSlice / 8), ax = (s >> 2) * 4 + (cls >> 2), az = (s & 3) * 4 + (cls & 3);
-                        reinterpret_cast<uint4*>(table)[e] =
-                            reinterpret_cast<const uint4*>(a.weights + (ax * 16 + az) * kSlice)[e % (kSlice / 8)];
-                    }
-                __syncthreads();
-                loaded = cls;
+            __syncthreads();
+            loaded = cls;
+        }
+        for (int64_t s = first + warp; s < last; s += kOneWarps) {
+            const int64_t bx = a.sites[s].center_x, bz = a.sites[s].center_z;
+            const int64_t ux0 = floor_div16(bx + lo) - 10, uz0 = floor_div16(bz + lo) - 10;
+            const int nx = (int)(floor_div16(bx + hi) + 10 - ux0 + 1);
+            const int nz = (int)(floor_div16(bz + hi) + 10 - uz0 + 1);
+            // Slime chunks (i, j) as i * kPad + j: lane = j, one i at a time.
+            const uint64_t xs = x_term((int32_t)(ux0 + lane)), zs = z_term((int32_t)(uz0 + lane)) + (uint64_t)a.seed;
+            int n = 0;
+            __syncwarp();
+            for (int i = 0; i < nx; ++i) {
+                const bool hit = slime_from_terms(__shfl_sync(0xFFFFFFFFu, xs, i), zs) && lane < nz;
+                const unsigned m = __ballot_sync(0xFFFFFFFFu, hit);
+                if (hit) list[warp][n + __popc(m & ((1u << lane) - 1u))] = (uint16_t)(i * kPad + lane);
+                n += __popc(m);
             }
-            for (int s = first; s < last; ++s) {
-                const int64_t bx = a.sites[s].center_x, bz = a.sites[s].center_z;
-                if ((int)(bx & 3) * 4 + (int)(bz & 3) != cls) continue;
-                const bool mine = done++ % kOneWarps == warp;
-                if (!mine) continue;
-                const int64_t ux0 = floor_div16(bx + lo) - 10, uz0 = floor_div16(bz + lo) - 10;
-                const int nx = (int)(floor_div16(bx + hi) + 10 - ux0 + 1);
-                const int nz = (int)(floor_div16(bz + hi) + 10 - uz0 + 1);
-                // Slime chunks (i, j) as i * kPad + j: lane = j, one i at a time.
-                const uint64_t xs = x_term((int32_t)(ux0 + lane)), zs = z_term((int32_t)(uz0 + lane)) + (uint64_t)a.seed;
-                int n = 0;
-                __syncwarp();
-                for (int i = 0; i < nx; ++i) {
-                    const bool hit = slime_from_terms(__shfl_sync(0xFFFFFFFFu, xs, i), zs) && lane < nz;
-                    const unsigned m = __ballot_sync(0xFFFFFFFFu, hit);
-                    if (hit) list[warp][n + __popc(m & ((1u << lane) - 1u))] = (uint16_t)(i * kPad + lane);
-                    n += __popc(m);
-                }
-                __syncwarp();
-                // This lane's offsets p = lane, lane + 32, lane + 64: first table entry of chunk (0, 0).
-                int base[3], obs[3] = {0, 0, 0};
+            __syncwarp();
+            // This lane's offsets p = lane, lane + 32, lane + 64: first table entry of chunk (0, 0).
+            int base[3], obs[3] = {0, 0, 0};
 #pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    const int p = min(lane + 32 * k, pairs - 1);
-                    const int64_t ox = bx + lo + (p / side) * 4, oz = bz + lo + (p % side) * 4;
-                    const int wx = (int)(floor_div16(ox) - 10 - ux0), wz = (int)(floor_div16(oz) - 10 - uz0);
-                    base[k] = (int)((((ox & 15) >> 2) * 4 + ((oz & 15) >> 2)) * kSlice) + (2 - wx) * kPad + 2 - wz;
-                }
+            for (int k = 0; k < 3; ++k) {
+                const int p = min(lane + 32 * k, pairs - 1);
+                const int64_t ox = bx + lo + (p / side) * 4, oz = bz + lo + (p % side) * 4;
+                const int wx = (int)(floor_div16(ox) - 10 - ux0), wz = (int)(floor_div16(oz) - 10 - uz0);
+                const int ax = (int)(ox & 15), az = (int)(oz & 15);
+                base[k] = (shared ? (ax >> 2) * 4 + (az >> 2) : ax * 16 + az) * kSlice + (2 - wx) * kPad + 2 - wz;
+            }
+            if (shared) {
 #pragma unroll 4
                 for (int c = 0; c < n; ++c) {
                     const int at = list[warp][c];
 #pragma unroll
                     for (int k = 0; k < 3; ++k) obs[k] += table[base[k] + at];
                 }
-                int best = -1, order = 0x7FFFFFFF;
+            } else {
+#pragma unroll 4
+                for (int c = 0; c < n; ++c) {
+                    const int at = list[warp][c];
 #pragma unroll
-                for (int k = 0; k < 3; ++k)
-                    if (lane + 32 * k < pairs && obs[k] > best) {  // offsets ascend: the first maximum wins
-                        best = obs[k];
-                        order = lane + 32 * k;
-                    }
-                const int top = __reduce_max_sync(0xFFFFFFFFu, best);
-                const int off = __reduce_min_sync(0xFFFFFFFFu, best == top ? order : 0x7FFFFFFF);
-                if (lane == 0) {
-                    ExtChunkResult& r = a.sites[s];
-                    const int y = top > 0 ? a.y_values[0] : a.platform_y;
-                    r.obs_count = a.pack_y ? (int32_t)((uint32_t)top | ((uint32_t)(y + 1024) << 20)) : top;
-                    r.afk_x = (int32_t)(top > 0 ? bx + lo + (off / side) * 4 : bx);
-                    r.afk_z = (int32_t)(top > 0 ? bz + lo + (off % side) * 4 : bz);
+                    for (int k = 0; k < 3; ++k) obs[k] += a.weights[base[k] + at];
                 }
+            }
+            int best = -1, order = 0x7FFFFFFF;
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                if (lane + 32 * k < pairs && obs[k] > best) {  // offsets ascend: the first maximum wins
+                    best = obs[k];
+                    order = lane + 32 * k;
+                }
+            const int top = __reduce_max_sync(0xFFFFFFFFu, best);
+            const int off = __reduce_min_sync(0xFFFFFFFFu, best == top ? order : 0x7FFFFFFF);
+            if (lane == 0) {
+                ExtChunkResult& r = a.sites[s];
+                const int y = top > 0 ? a.y_values[0] : a.platform_y;
+                r.obs_count = a.pack_y ? (int32_t)((uint32_t)top | ((uint32_t)(y + 1024) << 20)) : top;
+                r.afk_x = (int32_t)(top > 0 ? bx + lo + (off / side) * 4 : bx);
+                r.afk_z = (int32_t)(top > 0 ? bz + lo + (off % side) * 4 : bz);
             }
         }
     }
@@ -265,11 +271,11 @@ cudaError_t launch_precise(const PreciseArgs& a, cudaStream_t s) {
         // Sites per CTA and round: an even share of one wave, whole rounds of the CTA's warps from one
         // round on, and at most 256 (each thread looks at all of a chunk's alignments).
         constexpr int kCtas = 148 * 4;
-        int chunk = (a.n + kCtas - 1) / kCtas;
+        int64_t chunk = ((int64_t)a.n + kCtas - 1) / kCtas;
         if (chunk > kOneWarps) chunk = (chunk + kOneWarps - 1) / kOneWarps * kOneWarps;
         if (chunk > 256) chunk = 256;
-        const int grid = (a.n + chunk - 1) / chunk;
-        precise_one_kernel<<<grid < kCtas ? grid : kCtas, kOneTpb, 0, s>>>(a, chunk);
+        const int64_t grid = ((int64_t)a.n + chunk - 1) / chunk;
+        precise_one_kernel<<<(int)(grid < kCtas ? grid : kCtas), kOneTpb, 0, s>>>(a, (int)chunk);
         return cudaGetLastError();
     }
     const int grid = a.n < 148 * 16 ? a.n : 148 * 16;
