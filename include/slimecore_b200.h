@@ -137,11 +137,13 @@ void slime_b200_set_engine(int32_t mode, int32_t band_min_threshold);
  * band_min_periods x 2^17 chunks wide from band_min_threshold, or band_fast_periods x 2^17 wide from
  * band_fast_threshold; grouped bands (X phase pairs x groups of Z period copies) take areas
  * grouped_min_width chunks wide and wider (at most 16 x 2^17) from grouped_min_threshold: up to
- * grouped_max_width before the shared LCG, past it where neither of its branches applies. Of the others, thresholds below exact_below_threshold (on areas 2.25 x 2^17
- * chunks wide or more: below exact_wide_below_threshold) on areas of exact_min_centres centres or more
- * use the bit-plane kernels with exact counts (independent bands; from 2.25 x 2^17 grouped bands; from
- * 16 x 2^17 the shared LCG) while the expected number of sites stays below 1e9. Independent bands take
- * areas of indep_min_centres centres or more from indep_min_threshold; the general scan takes the rest.
+ * grouped_max_width before the shared LCG, past it where neither of its branches applies. Of the others,
+ * thresholds below exact_below_threshold (on areas 2.25 x 2^17 chunks wide or more: below
+ * exact_wide_below_threshold) on areas of exact_min_centres centres or more use the bit-plane kernels with
+ * exact counts: independent bands; from 2.25 x 2^17 (thresholds below 40: 4 x 2^17) grouped bands; from
+ * 16 x 2^17 the shared LCG; thin annuli at thresholds up to 40 the general scan. Independent
+ * bands take areas of indep_min_centres centres or more from indep_min_threshold; the general scan takes the
+ * rest, and every search with more than 4e9 expected sites (the band engines count into 32-bit bins).
  * Thresholds 28..222 (222 disables a branch;
  * exact_below_threshold and exact_wide_below_threshold 0..222, 0 disables them;
  * grouped_min_threshold 28..222), periods 2..64,

@@ -39,9 +39,14 @@ bool Context::ensure_band() {
 // shared-LCG band engine wants an area spanning two periods on one axis; the independent-band
 // engine wants enough centres to fill the GPU. The general scan takes the rest.
 int32_t Context::engine_for(const SearchSpec& q) const {
+    const int64_t w = 2 * q.rd_max + 1;
+    // The band engines count a whole search into 32-bit bins; beyond that the general scan, which counts each
+    // of its launches by itself (radius 1,250,000 with all sites in bins: threshold 40 3.6 s against 8.9).
+    constexpr double kBandMaxSites = 4e9;
+    if ((double)w * (double)w * tail_share(q.min_size) > kBandMaxSites) return kAlgoGeneral;
     if (engine_override == 4) return kAlgoBandExact;
     if (engine_override == 5) return kAlgoIndepExact;
-    const bool groups_fit = 2 * q.rd_max + 1 <= kGroupedMaxPeriods * kP;  // 16 copies at most
+    const bool groups_fit = w <= kGroupedMaxPeriods * kP;  // 16 copies at most
     if (engine_override == 7) return groups_fit ? kAlgoGroupedExact : kAlgoBandExact;
     if (engine_override == 1 || q.min_size < 28) return kAlgoGeneral;
     if (engine_override == 2) return kAlgoBand;
@@ -49,38 +54,37 @@ int32_t Context::engine_for(const SearchSpec& q) const {
     if (engine_override == 6) return groups_fit ? kAlgoGrouped : kAlgoBand;
     // The rule's numbers are measured crossovers (slime_b200/autotune.py writes them; the defaults are
     // the B200 values).
-    const int64_t w = 2 * q.rd_max + 1;
-    const bool wide = w >= kGroupedExactMinWidth, copies_fit = w <= kGroupedMaxPeriods * kP;
+    const bool wide = w >= kGroupedExactMinWidth;
     // Columns in words (bounded counts): shared LCG and grouped bands at high thresholds. Their
     // generator is cheaper than the bit planes', and few groups of windows pass its bounds there.
     const bool shared = (q.min_size >= band_min_threshold && w >= (int64_t)band_min_periods * kP) ||
                         (q.min_size >= band_fast_threshold && w >= (int64_t)band_fast_periods * kP);
     // Past grouped_max_width the shared LCG goes first; where its branches leave off, grouped bands go on
     // (radius 510,000, threshold 60: grouped 212 ms, shared 231 at 524,288, independent bands 513).
-    const bool grouped = q.min_size >= grouped_min_threshold && w >= grouped_min_width && copies_fit &&
+    const bool grouped = q.min_size >= grouped_min_threshold && w >= grouped_min_width && groups_fit &&
                          (w <= grouped_max_width || !shared);
-    // Bit planes (exact counts) below that, while the sites stay few enough to collect (the band
-    // engines emit every site in range; the general scan gates by count on the device). The generator's
-    // sharing and how full the words are decide the mode. B200, T centres/s at threshold 44: independent
-    // bands 1.60-1.68 at any width; grouped bands 1.26 / 1.64 / 1.74 / 2.22 / 3.41 at 1.5 / 2.3 / 3.1 /
-    // 4.6 / 15.3 periods; the shared LCG 1.54 / 2.43 / 2.86 at 9.2 / 15.3 / 19.1.
-    constexpr double kExactMaxSites = 1e9;
+    // Bit planes (exact counts) below that. The generator's sharing and how full the words are decide the
+    // mode. B200, T centres/s at threshold 44: independent bands 1.60-1.68 at any width; grouped bands 1.26 /
+    // 1.64 / 1.74 / 2.22 / 3.41 at 1.5 / 2.3 / 3.1 / 4.6 / 15.3 periods; the shared LCG 1.54 / 2.43 / 2.86 at
+    // 9.2 / 15.3 / 19.1.
     if (!shared && !grouped && q.min_size < (wide ? exact_wide_below_threshold : exact_below_threshold) &&
-        w * w >= exact_min_centres && (double)w * (double)w * tail_share(q.min_size) <= kExactMaxSites) {
+        w * w >= exact_min_centres) {
         const bool single = plane_union(q.min_size) == 1;  // every window counted by itself: thresholds below 40
         // Bit planes count all combos of a column at once, those inside the rd_min disc too; the general scan
         // skips the patches there. From these shares of the area outside the disc on down it is the faster one
-        // on wide areas at low thresholds. B200, inner radius 0.8 / 0.9 / 0.99 of the outer: radius 400,000,
-        // threshold 39 480 / 357 / 234 ms against 495 / 490 / 486; 900,000 at 40 2,382 / 1,772 / 1,161 against
-        // 1,694 / 1,692 / 1,690. Narrower areas and thresholds from 41 on lose nothing to the disc.
+        // at low thresholds. B200, inner radius 0.8 / 0.9 / 0.99 of the outer: radius 400,000, threshold 39 480 /
+        // 357 / 234 ms against 495 / 490 / 486; 900,000 at 40 2,382 / 1,772 / 1,161 against 1,694 / 1,692 / 1,690.
+        // Where more centres are kept, those inside the disc cost more: radius 300,000, threshold 35, 0.79 327
+        // against 380; 80,000 at 28, 0.7 45 against 57.
         const double outside = 1.0 - 3.14159265358979 * (double)q.rd_min * (double)q.rd_min / ((double)w * (double)w);
-        if (wide && outside < (single ? 0.5 : q.min_size == 40 ? 0.36 : 0.0)) return kAlgoGeneral;
+        const int t = q.min_size;
+        if (outside < (t < 30 ? 0.78 : t < 36 ? 0.6 : t < 40 ? 0.5 : t == 40 ? 0.36 : 0.0)) return kAlgoGeneral;
         // Single windows cost more to count than to generate, and grouped bands leave bits of a word empty:
         // they start at 4 periods there (radius 200,000, threshold 39 160 ms against 129 with independent
         // bands; 262,144: 218 against 221). Independent bands run the same kernels either way; counted by
         // unions of windows they are reported as bounded.
         if (!wide || (single && w < kGroupedSingleMinWidth)) return single ? kAlgoIndepExact : kAlgoIndep;
-        return copies_fit ? kAlgoGroupedExact : kAlgoBandExact;
+        return groups_fit ? kAlgoGroupedExact : kAlgoBandExact;
     }
     if (grouped) return kAlgoGrouped;
     if (shared) return kAlgoBand;

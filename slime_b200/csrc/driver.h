@@ -174,7 +174,7 @@ struct Context {
     int64_t indep_min_centres = 400040001;
     // Below exact_below_threshold (kGroupedExactMinWidth and wider: exact_wide_below_threshold), areas of
     // exact_min_centres centres or more that neither the shared LCG nor grouped bands take use the
-    // bit-plane kernels with exact counts, as long as the expected number of sites stays below 1e9.
+    // bit-plane kernels with exact counts.
     int32_t exact_below_threshold = 55;
     int64_t exact_min_centres = 400040001;
     // Grouped bands for areas of grouped_min_width chunks and more (at most kGroupedMaxPeriods periods) from

@@ -51,14 +51,15 @@ def test_arguments_out_of_range(core):
 
 def test_thin_annuli_of_low_thresholds_take_the_general_scan(core):
     pick = core.lib.slime_b200_engine_for
-    for r, threshold in ((147_456, 36), (200_000, 39), (400_000, 37), (690_000, 39), (150_000, 40), (900_000, 40)):
-        inside, outside = (0.75, 0.85) if threshold < 40 else (0.85, 0.95)
+    for r, threshold in ((10_000, 28), (80_000, 29), (20_011, 30), (300_000, 35), (10_000, 36), (20_011, 39), (100_000, 38),
+                         (147_456, 36), (200_000, 39), (400_000, 37), (690_000, 39), (150_000, 40), (900_000, 40)):
+        line = 0.529 if threshold < 30 else 0.714 if threshold < 36 else 0.798 if threshold < 40 else 0.903
+        inside, outside = line - 0.02, line + 0.02
         assert pick(r, threshold, int(outside * r)) == GENERAL
         assert pick(r, threshold, int(inside * r)) == pick(r, threshold, 0) != GENERAL
     for r in (147_456, 400_000, 900_000):
         for threshold in (41, 42, 50, 60):
             assert pick(r, threshold, r) == pick(r, threshold, 0) != GENERAL
-    assert pick(100_000, 39, 99_000) == pick(100_000, 39, 0) != GENERAL  # narrow areas stay
 
 
 def test_single_windows_of_narrow_areas_take_independent_bands(core):
@@ -66,3 +67,17 @@ def test_single_windows_of_narrow_areas_take_independent_bands(core):
     for r in (147_456, 200_000, 262_143):
         assert pick(r, 39, 0) == 310 and pick(r, 40, 0) == 230
     assert pick(262_144, 39, 0) == 230
+
+
+def test_only_more_sites_than_the_bins_hold_leave_the_band_engines(core):
+    """The band engines count a search into 32-bit bins, the general scan each of its launches."""
+    pick = core.lib.slime_b200_engine_for
+    assert pick(1_875_000, 40, 0) == pick(1_250_000, 40, 0) == 210  # 2.4e9 and 1.1e9 expected sites
+    assert pick(1_875_000, 39, 0) == GENERAL                       # 4.9e9
+    for mode in (2, 3, 4, 5, 6, 7):
+        core.lib.slime_b200_set_engine(mode, 0)
+        try:
+            assert pick(1_875_000, 39, 0) == pick(125_000, 0, 0) == GENERAL
+            assert pick(20_000, 40, 0) != GENERAL
+        finally:
+            core.lib.slime_b200_set_engine(0, 0)
