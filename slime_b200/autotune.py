@@ -3,8 +3,8 @@
     python -m slime_b200.autotune [--out slime_b200/tuning_b200.json] [--quick]
 
 For each (radius, threshold) point of a grid the search is timed with every engine that applies
-(the general scan, independent bands, grouped bands where the area spans a period, and the
-shared-LCG band engine where it spans two, all three also as bit planes), forced through slime_b200_set_engine; every engine
+(the general scan, independent bands, and as columns in words and as bit planes grouped bands where the area
+spans a period and the shared LCG where it spans two), forced through slime_b200_set_engine; every engine
 must return the same total and the same ranked sites. From the timings it derives the twelve
 numbers of slime_b200_set_engine_rule:
 
@@ -26,6 +26,7 @@ from __future__ import annotations
 import argparse
 import ctypes
 import json
+import math
 import time
 from pathlib import Path
 
@@ -50,49 +51,87 @@ def _time(core, mode, radius, thr, reps=2):
 
 GROUPED_MAX_PERIODS = 16  # grouped bands hold at most 16 period copies
 GROUPED_EXACT_MIN_WIDTH = 9 << 15  # the library's width from which bit planes run as grouped bands
+GROUPED_SINGLE_MIN_WIDTH = 4 << 17  # and below SINGLE_BELOW, where windows are counted one by one
+SINGLE_BELOW = 40
+# The bit planes' branch has the thresholds below; only a batch's small searches would follow the
+# independent bands' number there, and one alone is faster by the general scan (radius 2,000, threshold 40
+# 0.14 ms, as independent bands 0.30).
+INDEP_FROM = 42
+BAND_MAX_SITES = 4e9  # expected sites that the band engines count
+# On both sides of 8 and 16 periods, where a group more or less of copies fits a word.
+RADII = [10_000, 30_000, 100_000, 150_000, 200_000, 300_000, 450_000, 520_000, 530_000, 600_000, 1_000_000,
+         1_050_000, 1_250_000, 1_875_000]
+THRESHOLDS = [40, 42, 44, 46, 48, 50, 52, 53, 54, 55, 56, 58, 60]
+
+
+def tail_share(threshold):
+    """Expected share of centres whose count reaches the threshold (221 cells, one in ten)."""
+    return sum(math.comb(221, k) * 0.1**k * 0.9 ** (221 - k) for k in range(threshold, 222))
+
+
+TAIL = [tail_share(t) for t in range(223)]
+
+
+def engine(rule, width, threshold):
+    """The engine that the library's rule picks for a full square (Context::engine_for), by its name in the
+    timings; `rule` has the twelve numbers of slime_b200_set_engine_rule."""
+    bt, bp, ft, fp, it, ic, et, ec, gt, gw, gx, ew = rule
+    if width * width * TAIL[threshold] > BAND_MAX_SITES or threshold < 28:
+        return "general"
+    fits = width <= GROUPED_MAX_PERIODS * PERIOD
+    wide = width >= GROUPED_EXACT_MIN_WIDTH
+    shared = (threshold >= bt and width >= bp * PERIOD) or (threshold >= ft and width >= fp * PERIOD)
+    grouped = threshold >= gt and width >= gw and fits and (width <= gx or not shared)
+    if not shared and not grouped and threshold < (ew if wide else et) and width * width >= ec:
+        if not wide or (threshold < SINGLE_BELOW and width < GROUPED_SINGLE_MIN_WIDTH):
+            return "indep_exact" if threshold < SINGLE_BELOW else "indep"
+        return "grouped_exact" if fits else "band_exact"
+    if grouped:
+        return "grouped"
+    if shared:
+        return "band"
+    return "indep" if width * width >= ic and threshold >= it else "general"
 
 
 def measure(core, quick=False):
-    radii = [10_000, 30_000, 100_000, 150_000, 200_000, 300_000, 600_000] + ([] if quick else [1_000_000])
+    radii = [r for r in RADII if not quick or r <= 600_000]
     rows = []
     general_rate = {}
     for r in radii:
         w = 2 * r + 1
-        for thr in range(40, 62, 4 if quick else 2):
+        for thr in THRESHOLDS[:: 2 if quick else 1]:
             point = {"radius": r, "threshold": thr, "centres": w * w}
             ref = None
-            engines = []
-            if thr >= 42 or r <= 100_000:
-                engines += [("indep", 3)] + ([("band", 2)] if w >= 2 * PERIOD else [])
-                engines += [("grouped", 6)] if PERIOD < w <= GROUPED_MAX_PERIODS * PERIOD else []
-            engines += [("indep_exact", 5)] + ([("band_exact", 4)] if w >= 2 * PERIOD else [])
-            engines += [("grouped_exact", 7)] if PERIOD < w <= GROUPED_MAX_PERIODS * PERIOD else []
+            fits = w <= GROUPED_MAX_PERIODS * PERIOD
+            engines = [("indep_exact", 5)]
+            engines += [("band_exact", 4)] if w >= 2 * PERIOD else []
+            engines += [("grouped_exact", 7)] if PERIOD < w and fits else []
+            if thr >= 42 or r <= 100_000:  # bounded engines below 42 on large areas are never chosen
+                engines += [("band", 2)] if w >= 2 * PERIOD else []
+                engines += [("grouped", 6)] if PERIOD < w and fits else []
             if r <= 100_000:
                 engines.insert(0, ("general", 1))
             for name, mode in engines:
-                dt, out = _time(core, mode, r, thr, reps=1 if r >= 600_000 else 2)
+                dt, out = _time(core, mode, r, thr, reps=2)
                 if ref is None:
                     ref = out
                 elif out[0] != ref[0] or not np.array_equal(out[1], ref[1]):
                     raise RuntimeError(f"engines disagree at radius {r} threshold {thr}")
                 point[name + "_s"] = dt
+            point["indep_s"] = point["indep_exact_s"]  # the same kernels
             if "general_s" in point:
                 general_rate[thr] = point["centres"] / point["general_s"]
             else:
                 point["general_s"] = point["centres"] / general_rate.get(thr, min(general_rate.values()))
-            for k in ("indep", "band", "grouped"):  # bounded engines below 42 on large areas: never chosen
-                if k + "_s" not in point and (k == "indep" or (k == "band" and w >= 2 * PERIOD) or
-                                              (k == "grouped" and PERIOD < w <= GROUPED_MAX_PERIODS * PERIOD)):
-                    point[k + "_s"] = float("inf")
             rows.append(point)
     core.lib.slime_b200_set_engine(0, 0)
     return rows
 
 
 def planes_time(p):
-    """Time of the bit planes in the mode that the library picks for the point's width; None if not timed."""
+    """Time of the bit planes in the mode that the library picks for the point; None if not timed."""
     w = 2 * p["radius"] + 1
-    if w >= GROUPED_EXACT_MIN_WIDTH:
+    if w >= (GROUPED_SINGLE_MIN_WIDTH if p["threshold"] < SINGLE_BELOW else GROUPED_EXACT_MIN_WIDTH):
         for k in ("grouped_exact_s", "band_exact_s"):
             if k in p:
                 return p[k]
@@ -104,13 +143,25 @@ def planes_win(p):
     return planes_time(p) < min(p[k] for k in ("general_s", "band_s", "grouped_s") if k in p)
 
 
+def rule_time(p, rule):
+    """Time of a point under a rule: infinite where the rule picks an engine that was not timed there."""
+    name = engine(rule, 2 * p["radius"] + 1, p["threshold"])
+    if name.endswith("_exact"):
+        return planes_time(p) or math.inf
+    return p.get(name + "_s", math.inf)
+
+
+def best_time(p):
+    return min(v for k, v in p.items() if k.endswith("_s"))
+
+
 def derive(rows):
     """The rule numbers from the timings. Independent bands take a threshold when they beat
     the general scan there and at every higher measured threshold of the area. The two
     shared-LCG branches are chosen among the measured (threshold, periods) crossovers as the pair
     whose rule costs least over the whole grid (sum of each point's time over its best time), and
     the grouped-band branch (threshold, width range) is chosen the same way among the measured
-    thresholds and widths."""
+    thresholds and widths. The costs are those of the rule that the library runs (engine)."""
     def min_winning_thr(pts, a, b):
         pts = sorted(pts, key=lambda p: p["threshold"])
         best = 222
@@ -123,48 +174,42 @@ def derive(rows):
 
     by_r = {}
     for p in rows:
-        by_r.setdefault(p["radius"], []).append(p)
+        if p["threshold"] >= INDEP_FROM:
+            by_r.setdefault(p["radius"], []).append(p)
     indep_thr = {r: min_winning_thr(pts, "indep_s", "general_s") for r, pts in by_r.items()}
     indep_min_threshold = max(indep_thr.values())
     wins = [r for r, t in indep_thr.items() if t <= indep_min_threshold]
-    indep_min_centres = (2 * min(wins) + 1) ** 2 if wins else 1 << 62
-    cands = sorted({(p["threshold"], (2 * p["radius"] + 1) // PERIOD) for p in rows if "band_s" in p} | {(222, 64)})
+    indep = [indep_min_threshold, (2 * min(wins) + 1) ** 2 if wins else 1 << 62]
+    exact, wide = derive_exact(rows), derive_exact_wide(rows)
+    cands = sorted({(p["threshold"], max(2, (2 * p["radius"] + 1) // PERIOD)) for p in rows if "band_s" in p} | {(222, 64)})
     widths = sorted({2 * p["radius"] + 1 for p in rows if "grouped_s" in p})
     g_cands = [(t, lo, hi) for t in sorted({p["threshold"] for p in rows} | {222})
                for lo in widths for hi in widths if lo <= hi] or [(222, 1 << 40, 0)]
+    best = [best_time(p) for p in rows]
+
+    def numbers(a, b, g):
+        return [*a, *b, *indep, *exact, *g, wide]
 
     def cost(a, b, g):
-        total = 0.0
-        for p in rows:
-            w = 2 * p["radius"] + 1
-            planes = planes_time(p)
-            best = min([p[k] for k in ("general_s", "indep_s", "band_s", "grouped_s") if k in p] + ([planes] if planes else []))
-            thr = p["threshold"]
-            if "grouped_s" in p and thr >= g[0] and g[1] <= w <= g[2]:
-                t_rule = p["grouped_s"]
-            elif "band_s" in p and any(thr >= t and w >= n * PERIOD for t, n in (a, b)):
-                t_rule = p["band_s"]
-            else:
-                t_rule = p["indep_s"] if w * w >= indep_min_centres and thr >= indep_min_threshold else p["general_s"]
-                t_rule = min(t_rule, planes or t_rule)
-            total += t_rule / best
-        return total
+        rule = numbers(a, b, g)
+        return sum(rule_time(p, rule) / t for p, t in zip(rows, best))
 
     # Coordinate descent: the shared-LCG pair without grouped bands, the grouped triple given the
     # pair, then the pair again given the triple.
     g = (222, 1 << 40, 0)
-    a, b = min(((x, y) for x in cands for y in cands), key=lambda ab: cost(*ab, g))
+    pairs = [(x, y) for x in cands for y in cands if x <= y]
+    a, b = min(pairs, key=lambda ab: cost(*ab, g))
     g = min(g_cands, key=lambda gg: cost(a, b, gg))
-    a, b = min(((x, y) for x in cands for y in cands), key=lambda ab: cost(*ab, g))
-    return ([a[0], max(2, a[1]), b[0], max(2, b[1]), indep_min_threshold, indep_min_centres] + derive_exact(rows)
-            + [g[0], g[1], g[2], derive_exact_wide(rows)])
+    a, b = min(pairs, key=lambda ab: cost(*ab, g))
+    g = min(g_cands, key=lambda gg: cost(a, b, gg))
+    return numbers(a, b, g)
 
 
 def derive_exact(rows):
     """exact_below_threshold: one above the highest threshold at which the bit planes still beat every
     other branch on all areas of at least exact_min_centres centres, the smallest measured area where
-    they win at the lowest threshold."""
-    pts = [p for p in rows if "indep_exact_s" in p]
+    they win at the lowest threshold. (Wider areas have exact_wide_below_threshold.)"""
+    pts = [p for p in rows if "indep_exact_s" in p and 2 * p["radius"] + 1 < GROUPED_EXACT_MIN_WIDTH]
     if not pts:
         return [0, 1 << 62]
     lowest = min(p["threshold"] for p in pts)
@@ -183,13 +228,14 @@ def derive_exact(rows):
 
 
 def derive_exact_wide(rows):
-    """exact_wide_below_threshold: one above the highest threshold up to which the bit planes beat
-    every other branch on every measured area at least GROUPED_EXACT_MIN_WIDTH wide."""
+    """exact_wide_below_threshold: one above the highest threshold up to which the bit planes beat every
+    other branch on some measured area at least GROUPED_EXACT_MIN_WIDTH wide: the library asks the other
+    branches first, so that they keep the areas where they win."""
     pts = [p for p in rows if "indep_exact_s" in p and 2 * p["radius"] + 1 >= GROUPED_EXACT_MIN_WIDTH]
     below = 0
     for thr in sorted({p["threshold"] for p in pts}):
         at = [p for p in pts if p["threshold"] == thr]
-        if all(planes_win(p) for p in at):
+        if any(planes_win(p) for p in at):
             below = thr + 1
         else:
             break

@@ -166,7 +166,7 @@ struct Context {
     // from band_fast_threshold; independent bands for areas of indep_min_centres centres or more
     // from indep_min_threshold; the general scan otherwise. Defaults: B200 measurements
     // (slime_b200/tuning_b200.json).
-    int32_t band_min_threshold = 53;
+    int32_t band_min_threshold = 54;
     int32_t band_min_periods = 16;
     int32_t band_fast_threshold = 55;
     int32_t band_fast_periods = 8;
@@ -175,14 +175,14 @@ struct Context {
     // Below exact_below_threshold (kGroupedExactMinWidth and wider: exact_wide_below_threshold), areas of
     // exact_min_centres centres or more that neither the shared LCG nor grouped bands take use the
     // bit-plane kernels with exact counts.
-    int32_t exact_below_threshold = 55;
+    int32_t exact_below_threshold = 57;
     int64_t exact_min_centres = 400040001;
     // Grouped bands for areas of grouped_min_width chunks and more (at most kGroupedMaxPeriods periods) from
     // grouped_min_threshold; past grouped_max_width only where the shared LCG's branches do not apply.
-    int32_t grouped_min_threshold = 55;
-    int32_t exact_wide_below_threshold = 55;
+    int32_t grouped_min_threshold = 56;
+    int32_t exact_wide_below_threshold = 56;
     int64_t grouped_min_width = 200001;
-    int64_t grouped_max_width = 1000001;
+    int64_t grouped_max_width = 200001;
     int64_t last_rare = 0;             // rare redraw chunks found by the last band search
     uint32_t wait_polls = 1u << 22;    // bounded mbarrier waits of the band kernels
 

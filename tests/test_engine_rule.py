@@ -29,7 +29,7 @@ def test_wide_areas_always_share_the_generator(core):
 
 
 def test_grouped_bands_go_on_to_the_shared_lcg(core):
-    for threshold in (55, 60, 75):
+    for threshold in (56, 60, 75):
         for r in (500_000, 500_001, 510_000, 524_287):
             assert core.lib.slime_b200_engine_for(r, threshold, 0) == GROUPED
         assert core.lib.slime_b200_engine_for(524_288, threshold, 0) == SHARED
