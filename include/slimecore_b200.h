@@ -166,6 +166,12 @@ void slime_b200_set_tuning(int32_t band_mad_add);
  * first wait gives up at once. */
 int64_t slime_b200_set_wait_limit(int64_t polls);
 
+/* Adjacent windows that the bit-plane kernels count as one: 1, 2 or 4; 0 restores the choice by threshold.
+ * Results are identical. Returns the previous value, or -1 for another number (nothing is changed). For
+ * tests: counted by twos or fours at low thresholds, far more unions reach the threshold than the kernels'
+ * lists hold. */
+int32_t slime_b200_set_plane_union(int32_t joined);
+
 /* Last CUDA error text of this library ("" if none). */
 const char* slime_b200_last_error(void);
 

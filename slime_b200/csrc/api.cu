@@ -679,6 +679,14 @@ int64_t slime_b200_set_wait_limit(int64_t polls) {
     return before;
 }
 
+int32_t slime_b200_set_plane_union(int32_t joined) {
+    if (joined != 0 && joined != 1 && joined != 2 && joined != 4) return -1;
+    std::lock_guard<std::mutex> lock(ctx().mu);
+    const int32_t before = ctx().plane_union_override;
+    ctx().plane_union_override = joined;
+    return before;
+}
+
 void slime_b200_set_engine(int32_t mode, int32_t band_min_threshold) {
     std::lock_guard<std::mutex> lock(ctx().mu);
     ctx().engine_override = (mode >= 0 && mode <= 7) ? mode : 0;

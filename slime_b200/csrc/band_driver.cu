@@ -180,8 +180,7 @@ cudaError_t launch_band_scan(const BandArgs& a, int grid, cudaStream_t s) {
 int band_class(const BandArgs& a) {
     const int mode = band_mode(a);
     if (!band_planes(mode, a.exact != 0)) return (mode == kBandGrouped ? 2 : 0) + (band_keeps_candidates(a.min_size) ? 1 : 0);
-    const int joined = plane_union(a.min_size);
-    return 4 + 3 * mode + (joined == 4 ? 2 : joined - 1);
+    return 4 + 3 * mode + (a.joined == 4 ? 2 : a.joined - 1);
 }
 
 bool Context::scan_band(const SearchSpec& q, std::vector<Hit>& best, Counts& h,
@@ -309,6 +308,7 @@ bool Context::scan_band(const SearchSpec& q, std::vector<Hit>& best, Counts& h,
                 a.indep = indep ? 1 : 0;
                 a.groups = G.groups;
                 a.exact = exact ? 1 : 0;
+                a.joined = joined_windows(q.min_size);
                 a.one = 1u;
                 a.poll_limit = wait_polls;
                 a.hist = dhist;

@@ -85,7 +85,7 @@ cudaError_t run_band_items(std::vector<BandArgs>& items, BandArgs* args_dev, int
         while (i1 < m && band_class(items[i1]) == cls) ++i1;
         const int grid = band_grid(planes, sm_count);
         const int32_t n = (int32_t)(i1 - i0);
-        e = planes ? launch_plane_batch(args_dev + i0, prefix_dev + i0, n, heads_dev + cls, mode, plane_union(items[i0].min_size), grid, s)
+        e = planes ? launch_plane_batch(args_dev + i0, prefix_dev + i0, n, heads_dev + cls, mode, items[i0].joined, grid, s)
                    : launch_column_batch(args_dev + i0, prefix_dev + i0, n, heads_dev + cls, mode,
                                          band_keeps_candidates(items[i0].min_size), grid, s);
         if (e != cudaSuccess) return e;
@@ -262,6 +262,7 @@ int32_t Context::search_batch(const SearchSpec* reqs, int32_t n, ExtChunkResult*
             a.emitted = bt_counts.ptr + 2 * s;
             a.overflow = bt_flags.ptr + 4 * s;
             a.exact = p.exact ? 1 : 0;
+            a.joined = joined_windows(q.min_size);
             a.one = 1u;
             a.poll_limit = wait_polls;
             a.indep = g.indep ? 1 : 0;

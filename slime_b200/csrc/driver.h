@@ -185,6 +185,8 @@ struct Context {
     int64_t grouped_max_width = 200001;
     int64_t last_rare = 0;             // rare redraw chunks found by the last band search
     uint32_t wait_polls = 1u << 22;    // bounded mbarrier waits of the band kernels
+    int32_t plane_union_override = 0;  // slime_b200_set_plane_union
+    int joined_windows(int32_t min_size) const { return plane_union_override ? plane_union_override : plane_union(min_size); }
 
     // Y-scan configuration (set_y_scan_config) and the tables built from it.
     int32_t y_enabled = 0, platform_y = -64, y_min = -64, y_max = 64, y_step = 4;

@@ -92,7 +92,7 @@ struct BandArgs {
     int64_t row_stride;      // input rows between band j and band j + 1 (2^17 with the shared LCG;
                              // grouped bands: between group g and group g + 1)
     int32_t groups;          // grouped bands (G > 0): G groups of nb / G copies 2^17 apart
-    int32_t pad_;
+    int32_t joined;          // bit planes: adjacent windows counted as one (1, 2 or 4)
 };
 
 // Tiling of one band search (band_driver.cu): axes (u = phase axis, v = band axis), phases,

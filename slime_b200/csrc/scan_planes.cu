@@ -88,7 +88,7 @@ cudaError_t launch_plane_batch(const BandArgs* args, const int64_t* prefix, int3
 }
 
 cudaError_t launch_plane_scan(const BandArgs& a, int grid, cudaStream_t s) {
-    return run_planes(band_mode(a), plane_union(a.min_size), a, nullptr, nullptr, 0, nullptr, grid, s);
+    return run_planes(band_mode(a), a.joined, a, nullptr, nullptr, 0, nullptr, grid, s);
 }
 
 cudaError_t launch_plane_row_terms(uint32_t* rt, int32_t vrows_alloc, int32_t vrows, int32_t nj, int32_t row_first,

@@ -364,6 +364,7 @@ bool Server::step(std::vector<Job*>& live) {
         a.emitted = j->counts;
         a.overflow = j->flags;
         a.exact = j->exact ? 1 : 0;
+        a.joined = c.joined_windows(q.min_size);
         a.one = 1u;
         a.poll_limit = c.wait_polls;
         a.indep = g.indep ? 1 : 0;
