@@ -100,8 +100,11 @@ void plan_job(Job& j, const Context& c) {
     // Whatever the inner radius: a general scan would hold every other request for its whole length.
     SearchSpec full = q;
     full.rd_min = 0;
-    const int32_t algo = c.engine_for(full);
+    int32_t algo = c.engine_for(full);
     const double centres = (double)W * (double)W;
+    // Searches of low thresholds with more than 1e9 sites run whole, with the memory of a single search: a
+    // budget too small for that keeps refusing them.
+    if (q.min_size < 42 && centres * tail_share(q.min_size) > 1e9) algo = kAlgoGeneral;
     // Emission gate, as the single search chooses it (biome requests keep more, as there).
     const int64_t want = (q.biome_flags & 3) ? 2LL * q.max_results + 1024 : (int64_t)q.max_results;
     const int32_t emit = emission_gate(q, want);
