@@ -25,6 +25,10 @@ REF_SO = HERE / "_ref" / "libslimecore_ref.so"
 REF_GPU_SO = HERE / "_ref" / "libslimecore_gpu_ref.so"
 
 
+class ReferenceNotBuilt(FileNotFoundError):
+    """A reference library is absent: its source tree was not there when the checkers were built."""
+
+
 def reference_dir(ref_dir=None):
     """The reference source tree: the argument, else $SLIME_REFERENCE_DIR, else None (no default)."""
     d = ref_dir if ref_dir is not None else os.environ.get("SLIME_REFERENCE_DIR")
@@ -136,7 +140,7 @@ class RefCpu:
 
     def __init__(self, path: Path = REF_SO):
         if not Path(path).exists():
-            raise FileNotFoundError(f"{path} is not built (needs the reference source tree)")
+            raise ReferenceNotBuilt(f"{path} is not built (needs the reference source tree)")
         lib = C.CDLL(str(path))
         i64, i32, vp = C.c_int64, C.c_int32, C.c_void_p
         lib.search_slime_clusters_centered.argtypes = [i64, i64, i32, i32, i64, i32, i32, vp,
@@ -195,7 +199,7 @@ class RefGpu:
 
     def __init__(self, path: Path = REF_GPU_SO):
         if not Path(path).exists():
-            raise FileNotFoundError(f"{path} is not built (needs the reference source tree)")
+            raise ReferenceNotBuilt(f"{path} is not built (needs the reference source tree)")
         lib = C.CDLL(str(path))
         i64, i32, vp = C.c_int64, C.c_int32, C.c_void_p
         lib.search_slime_clusters_gpu_v1_centered.argtypes = [i64, i64, i32, i32, i64, i32, i32,
@@ -323,7 +327,7 @@ class RefBiomeHost(_BiomeCalls):
 
     def __init__(self, path: Path = REF_BIOME_HOST_SO):
         if not Path(path).exists():
-            raise FileNotFoundError(f"{path} is not built (needs the reference source tree)")
+            raise ReferenceNotBuilt(f"{path} is not built (needs the reference source tree)")
         self._bind(C.CDLL(str(path)), "refb_")
 
 
@@ -334,7 +338,7 @@ class RefBiomeGpu:
     def __init__(self, kind: str = "nofmad"):
         path = REF_BIOME_GPU_SO[kind]
         if not path.exists():
-            raise FileNotFoundError(f"{path} is not built (needs the reference source tree)")
+            raise ReferenceNotBuilt(f"{path} is not built (needs the reference source tree)")
         lib = C.CDLL(str(path))
         vp, i32, u64 = C.c_void_p, C.c_int32, C.c_uint64
         lib.mcgpu_modern_ctx_create.argtypes = [i32, u64, i32]
