@@ -134,8 +134,9 @@ def strip_tiles(rows: int = STRIP_ROWS):
 
 
 def cpu_strip(seed: int, rows: int = STRIP_ROWS):
-    """Reference CPU library (SlimeCore.cpp, AVX2 + OpenMP, all host threads) over the fixed
-    full-width strip of the threshold-60 workload; returns T centres/s and the sample info."""
+    """Reference CPU library (SlimeCore.cpp, AVX2 + OpenMP, all host threads; kind "reference") over
+    the fixed full-width strip of the threshold-60 workload, or where it is not built the oracle's C
+    restatement (kind "port"); returns T centres/s and the sample info."""
     from oracle.oracle import REF_SO, RefCpu, Oracle
     threads = os.cpu_count() or 1
     if REF_SO.exists():
@@ -157,12 +158,17 @@ def cpu_strip(seed: int, rows: int = STRIP_ROWS):
 
 
 def cpu_baseline(seed: int):
-    """The reported CPU baseline of our arm: the reference CPU library on the fixed strip."""
+    """The reported CPU baseline of our arm, on the fixed strip."""
     return cpu_strip(seed)
 
 
 def run_reference(args, rank, world):
     if rank != 0:
+        return
+    from oracle.oracle import REF_SO
+    if not REF_SO.exists():
+        print(json.dumps({"impl": "reference", "unavailable":
+                          f"{REF_SO.name} is not built: the reference's source tree was absent"}), flush=True)
         return
     spec = workloads.full_world_scan()
     vals = []
