@@ -141,7 +141,8 @@ void slime_b200_set_engine(int32_t mode, int32_t band_min_threshold);
  * thresholds below exact_below_threshold (on areas 2.25 x 2^17 chunks wide or more: below
  * exact_wide_below_threshold) on areas of exact_min_centres centres or more use the bit-plane kernels with
  * exact counts: independent bands; from 2.25 x 2^17 (thresholds below 40: 4 x 2^17) grouped bands; from
- * 16 x 2^17 the shared LCG; thin annuli at thresholds up to 40 the general scan. Independent
+ * 16 x 2^17 the shared LCG; thin annuli at thresholds up to 40, and searches whose
+ * upper bound leaves many sites at the best count, the general scan. Independent
  * bands take areas of indep_min_centres centres or more from indep_min_threshold; the general scan takes the
  * rest, and every search with more than 4e9 expected sites (the band engines count into 32-bit bins).
  * Thresholds 28..222 (222 disables a branch;

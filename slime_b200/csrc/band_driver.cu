@@ -79,6 +79,13 @@ int32_t Context::engine_for(const SearchSpec& q) const {
         const double outside = 1.0 - 3.14159265358979 * (double)q.rd_min * (double)q.rd_min / ((double)w * (double)w);
         const int t = q.min_size;
         if (outside < (t < 30 ? 0.78 : t < 36 ? 0.6 : t < 40 ? 0.5 : t == 40 ? 0.36 : 0.0)) return kAlgoGeneral;
+        // An upper bound can stop the emission gate at a count that many centres share, and a site sent costs
+        // more here (its filter against the redrawn chunks, launches cut to the hit buffer) than in the general
+        // scan: by the share of the centres sent, 1.2e-3 (radius 100,000, counts 30 to 36) 582 ms against 310,
+        // 1.8e-4 (1,000,000, 39) 10.9 s against 9.3, 8.9e-5 (1,250,000, 40) 9.3 against 12.1.
+        if (q.max_size < kHistBins - 1 &&
+            tail_share(emission_gate(q, q.max_results)) - tail_share(q.max_size + 1) > 1.3e-4)
+            return kAlgoGeneral;
         // Single windows cost more to count than to generate, and grouped bands leave bits of a word empty:
         // they start at 4 periods there (radius 200,000, threshold 39 160 ms against 129 with independent
         // bands; 262,144: 218 against 221). Independent bands run the same kernels either way; counted by

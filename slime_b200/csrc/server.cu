@@ -97,9 +97,11 @@ namespace {
 void plan_job(Job& j, const Context& c) {
     const SearchSpec& q = j.q;
     const int64_t W = 2 * q.rd_max + 1;
-    // Whatever the inner radius: a general scan would hold every other request for its whole length.
+    // Whatever the inner radius and the upper bound: a general scan would hold every other request for its
+    // whole length.
     SearchSpec full = q;
     full.rd_min = 0;
+    full.max_size = kHistBins - 1;
     int32_t algo = c.engine_for(full);
     const double centres = (double)W * (double)W;
     // Searches of low thresholds with more than 1e9 sites run whole, with the memory of a single search: a

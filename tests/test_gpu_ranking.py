@@ -50,3 +50,18 @@ def test_more_sites_at_the_gate_than_the_hit_buffer_holds(core, radius, low, hig
             core.lib.slime_b200_set_engine(0, 0)
     assert results[0][0] == results[1][0]
     assert np.array_equal(results[0][1], results[1][1])
+
+
+@pytest.mark.parametrize("low,high,engine", [(30, 33, 100), (36, 37, 100), (39, 221, 310), (40, 44, 300), (45, 45, 300)])
+def test_searches_that_send_many_sites_take_the_general_scan(core, low, high, engine):
+    """Radius 12,000: an upper bound that leaves many sites at the best count (0.6 % and 0.06 % of the centres),
+    and bounds that do not."""
+    total, got = core.search(77, 12_000, low, high, 0, 1_000, -1_000, 500)
+    assert core.lib.get_gpu_v1_algorithm() == engine
+    core.lib.slime_b200_set_engine(5, 0)
+    try:
+        total5, got5 = core.search(77, 12_000, low, high, 0, 1_000, -1_000, 500)
+    finally:
+        core.lib.slime_b200_set_engine(0, 0)
+    assert total == total5
+    assert np.array_equal(got, got5)
