@@ -7,6 +7,7 @@ loudly (the search returns -1 and :class:`SlimeCoreB200` raises).
 from __future__ import annotations
 
 import ctypes as C
+import json
 from pathlib import Path
 
 import numpy as np
@@ -133,6 +134,12 @@ RULE_KEYS = ("band_min_threshold", "band_min_periods", "band_fast_threshold", "b
              "grouped_min_threshold", "grouped_min_width", "grouped_max_width", "exact_wide_below_threshold")
 
 
+def tuned_rule(path: Path = TUNING) -> dict:
+    """The engine rule of a tuning file, without decoding the timings beside it."""
+    text = path.read_text()
+    return json.JSONDecoder().raw_decode(text, text.index("{", text.index('"rule"')))[0]
+
+
 class SlimeCoreB200:
     """Pythonic view of the C ABI; every call goes through the exported C functions. The engine
     rule measured by slime_b200/autotune.py (tuning_b200.json) is applied when present."""
@@ -140,8 +147,7 @@ class SlimeCoreB200:
     def __init__(self, path: Path | str = LIB, apply_tuning: bool = True):
         self.lib = load(path)
         if apply_tuning and TUNING.exists():
-            import json
-            self.set_engine_rule(json.loads(TUNING.read_text())["rule"])
+            self.set_engine_rule(tuned_rule())
 
     def set_engine_rule(self, rule: dict):
         keys = next(RULE_KEYS[:n] for n in (12, 8, 6) if all(k in rule for k in RULE_KEYS[:n]))

@@ -70,3 +70,17 @@ def test_the_tuner_scores_the_rule_that_the_library_runs(core):
     finally:
         core.set_engine_rule(before)
     assert PERIOD == 1 << 17
+
+
+def test_the_binding_reads_the_rule_of_the_file(doc, core, tmp_path):
+    from slime_b200.lib import SlimeCoreB200, tuned_rule
+    assert tuned_rule() == doc["rule"]
+    other = tmp_path / "rule.json"
+    other.write_text(json.dumps({"rule": dict(doc["rule"], band_min_threshold=60), "points": []}, indent=2))
+    assert tuned_rule(other) == dict(doc["rule"], band_min_threshold=60)
+    before = core.engine_rule()
+    try:
+        core.set_engine_rule(dict(before, band_min_threshold=60))
+        assert SlimeCoreB200().engine_rule() == doc["rule"]
+    finally:
+        core.set_engine_rule(before)
