@@ -122,7 +122,7 @@ int64_t slime_b200_last_rare_chunks(void);
  * 3 the independent-band engine and 6 the grouped-band engine whenever the threshold allows it
  * (min_size >= 28), 4 / 5 / 7 the shared-LCG / independent-band / grouped-band engine with
  * bit-sliced counts of every centre (any threshold). Grouped modes wider than 16 x 2^17 chunks run as the
- * shared LCG.
+ * shared LCG, and searches with more than 4e9 expected sites as the general scan in every mode.
  * `band_min_threshold` (28..221, other values keep the current one) is the smallest threshold
  * automatic mode sends to the shared-LCG band engine. Results are identical either way; only
  * speed differs. get_gpu_v1_algorithm() reports 100 (general), 200 (band), 300 (independent

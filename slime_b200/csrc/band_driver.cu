@@ -35,9 +35,9 @@ bool Context::ensure_band() {
     return true;
 }
 
-// Engine choice. The band engines need a threshold >= 28 (their byte-lane bound test). The
-// shared-LCG band engine wants an area spanning two periods on one axis; the independent-band
-// engine wants enough centres to fill the GPU. The general scan takes the rest.
+// Engine choice. The automatic rule uses the band engines from threshold 28 on (the byte-lane bound test of
+// the columns in words needs that). The shared LCG wants an area of many periods; the independent bands want
+// enough centres to fill the GPU. The general scan takes the rest.
 int32_t Context::engine_for(const SearchSpec& q) const {
     const int64_t w = 2 * q.rd_max + 1;
     // The band engines count a whole search into 32-bit bins; beyond that the general scan, which counts each
@@ -136,8 +136,8 @@ BandGeom band_geometry(int64_t W, int64_t H, int mode, bool planes, int sm_count
     g.pairs = (g.nI + 1) / 2;
     // Tile height: the tiles of a launch run in waves of `slots` CTAs, each tile 16 halo rows taller
     // than its centres. The height (at most 2,048 rows) whose waves take the fewest rows wins; with
-    // many waves the last one hardly counts. (Radius 20,011, 40 columns of tiles: 8 tiles high made
-    // 320 tiles on 148 CTAs, 3 waves of 173 rows where 7 make 2 of 195.)
+    // many waves the last one hardly counts. (Radius 20,011, 40 columns of tiles of the bit planes: 8 tiles
+    // high would be 320 tiles on 296 CTAs, 2 waves of 173 rows where 7 make one of 195.)
     const int64_t slots = band_grid(planes, sm_count), columns = g.u_tiles * g.pairs;
     int64_t best_vt = 0;
     double best_rows = 0;

@@ -109,9 +109,9 @@ constexpr int kBandShared = 0, kBandIndep = 1, kBandGrouped = 2;
 // Tiling of a search area; `planes` says which kernels run it (band_planes).
 BandGeom band_geometry(int64_t W, int64_t H, int mode, bool planes, int sm_count);
 
-// Two kernel families share BandArgs. scan_band.cu: a word holds 32 columns of one combo (bounded
-// counts of shared and grouped bands). planes.cuh: a word holds 32 combos of one column (exact counts,
-// and independent bands).
+// Two kernel families share BandArgs. scan_band.cu: a word holds 32 columns of one combo (shared and
+// grouped bands at high thresholds, bounded counts). planes.cuh: a word holds 32 combos of one column (the same
+// modes at lower thresholds, and independent bands).
 inline bool band_planes(int mode, bool exact) { return exact || mode == kBandIndep; }
 inline int band_mode(const BandArgs& a) { return a.indep ? kBandIndep : a.groups ? kBandGrouped : kBandShared; }
 int band_max_bands();

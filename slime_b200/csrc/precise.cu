@@ -14,7 +14,7 @@
 //    site: it lists the slime chunks of the 23 x 23 that any offset reaches, and each lane adds up
 //    the entries of its three offsets. Per chunk that is one broadcast and three lookups a warp; a CTA
 //    per site with the table in global memory spent its time on 44 dependent steps of bit scanning a
-//    lane and eight block barriers a site. 20,000 sites: 243 -> 86 us (issue slots 56 % busy).
+//    lane and eight block barriers a site. 20,000 sites: 243 -> 69 us (issue slots 65 % busy).
 //  * Several Y levels (precise_kernel): one CTA per site builds the 23 x 23 bitmap once; threads split the
 //    (offset, Y) pairs, neighbours in Y, so the table reads coalesce; a block reduction picks (max obs,
 //    first order).

@@ -58,9 +58,10 @@ int plane_row_words(int mode) { return mode == kBandShared ? kRowWordsS : kRowWo
 // Per four columns and row a warp issues about 336, 170 or 90 adders for unions of 1, 2 or 4 windows and
 // 90 instructions for each union of its 1,024 x (4 / kUnion) that reaches the threshold (binomial tails of
 // 238 and 272 cells: 8e-4 and 9e-3 at 40, 5e-5 and 1e-3 at 44). Measured, radius 100,000, independent
-// bands, with 1 / 2 / 4: threshold 40 33.7 / 33.8 / 87.9 ms, 42 30.9 / 27.1 / 47.1, 46 30.0 / 24.2 / 26.2,
-// 48 29.9 / 23.9 / 24.4, 60 29.9 / 23.8 / 23.3; radius 300,000, grouped bands: 46 219 / 154.6 / 156.7,
-// 48 218 / 152 / 141.
+// bands, with 1 / 2 / 4: threshold 39 33.5 / 40.0 ms, 40 31.1 / 32.4 / 85.1, 42 28.3 / 25.5 / 44.4, 46 27.6 /
+// 22.6 / 23.4, 47 27.6 / 22.4 / 22.3, 60 27.5 / 22.2 / 20.6; radius 300,000, grouped bands: 38 313 / 432, 40 266 /
+// 240 / 727, 46 216 / 153 / 155, 47 216 / 151 / 145; radius 1,250,000, shared LCG: 46 3,339 / 2,052 / 2,078, 48
+// 3,332 / 2,015 / 1,783.
 constexpr int kUnionTwoFrom = 40, kUnionFourFrom = 47;
 int plane_union(int min_size) { return min_size >= kUnionFourFrom ? 4 : min_size >= kUnionTwoFrom ? 2 : 1; }
 
