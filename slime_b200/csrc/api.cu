@@ -193,7 +193,7 @@ void rank_best(std::vector<Hit>& v, const Counts& h, const SearchSpec& q, size_t
         if (packed) other.resize(n);
     } catch (const std::bad_alloc&) {  // no room beside the hits: sort them in place
     }
-    if (other.size() < n) {
+    if (!packed || other.size() < n) {
         std::sort(v.begin(), v.end(), hit_better);
         return;
     }
