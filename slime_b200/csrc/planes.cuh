@@ -95,10 +95,9 @@ struct __align__(16) PlaneSmem {
     uint32_t list[kListCap];                  // unions waiting for their windows' counts
     unsigned int listed;
     unsigned int hist[kHistBins];             // counts of this CTA's centres in range (if args.hist)
-    // Of the current tile's search, by band: first area row (before the tile's base row), and with grouped
-    // bands the base row from which its rows belong to the next copy's first group.
-    int64_t row0[kMaxBands];
-    int32_t row_end[kGrpBands];
+    // Grouped bands, of the current tile's search, by band: first area row (before the tile's base row), and
+    // the base row from which its rows belong to the next copy's first group.
+    int32_t row0[kGrpBands], row_end[kGrpBands];
 };
 static_assert(sizeof(PlaneSmem) <= (233472 - 2048) / kCtasPerSm, "two CTAs an SM");
 
@@ -388,7 +387,7 @@ __device__ __forceinline__ void keep_centre(PlaneSmem& S, const BandArgs& a, con
     if (m >= a.nb || c < 0 || c >= Shape<kMode>::kOutW || rr < 0 || rr >= T.out_h) return;
     const int64_t u = (int64_t)T.u0 + c;
     const int64_t cu = u + (int64_t)(T.i0 + ph) * kPeriod;
-    const int64_t cv = (int64_t)T.v0 + rr + S.row0[m];
+    const int64_t cv = (int64_t)T.v0 + rr + (kMode == kModeGrouped ? (int64_t)S.row0[m] : (a.j0 + m) * a.row_stride);
     if (kMode == kModeGrouped && T.v0 + rr >= S.row_end[m]) return;
     if (u >= a.ubase || cu >= a.width_u || cv >= a.height_v) return;
     const int32_t cx = (int32_t)(a.transposed ? a.area_x0 + cv : a.area_x0 + cu);
@@ -697,11 +696,10 @@ __device__ __forceinline__ bool plane_tile(PlaneSmem& S, const BandArgs& a, int6
     for (int i = tid; i < kRingWords / 4; i += kTpb) reinterpret_cast<uint4*>(S.ring)[i] = make_uint4(0u, 0u, 0u, 0u);
     // Worked out a kept centre at a time, the bands' rows cost five divisions each: grouped bands at thresholds
     // below 40 took up to twice as long (radius 180,000, threshold 37: 252 ms).
-    if (tid < kMaxBands) {
+    if (kMode == kModeGrouped && tid < kGrpBands) {
         const int copy = tid % T.copies, group = tid / T.copies;
-        S.row0[tid] = kMode == kModeGrouped ? copy * kPeriod + group * a.row_stride : (a.j0 + tid) * a.row_stride;
-        if (kMode == kModeGrouped && tid < kGrpBands)
-            S.row_end[tid] = T.copies > 1 ? (int32_t)max((int64_t)0, kPeriod - group * a.row_stride) : INT32_MAX;
+        S.row0[tid] = copy * (int32_t)kPeriod + group * (int32_t)a.row_stride;
+        S.row_end[tid] = T.copies > 1 ? max(0, (int32_t)kPeriod - group * (int32_t)a.row_stride) : INT32_MAX;
     }
     // Row terms of batches 0 and 1 (batch b lives in rows[b % 2]).
     if (tid == 0) {
