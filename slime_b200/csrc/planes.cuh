@@ -19,8 +19,8 @@
 //    one count then stands for 1, 2 or 4 columns. A union that reaches the threshold is looked at by
 //    the whole warp, which counts its windows one by one.
 // What bounds it (B200): integer issue. Independent bands, radius 100,000: the generator is about 18 ms
-// (13.9 cycles a warp test in a probe of it alone); with the counter 25.5 ms at threshold 42, 23.4 at 44 and
-// 20.6 at 60. Packing columns took 42.4 ms at threshold 42 and 29.3 at 60. Grouped bands, radius 300,000,
+// (13.9 cycles a warp test in a probe of it alone); with the counter 25.5 ms at threshold 42, 23.3 at 44 and
+// 20.8 at 60. Packing columns took 42.4 ms at threshold 42 and 29.3 at 60. Grouped bands, radius 300,000,
 // threshold 44: 160 against 276 ms, threshold 50 (there bounded): 133 against 183 ms.
 // Shared and grouped bands at high thresholds stay with columns in words (radius 1,250,000, threshold 60:
 // 1,012 ms; radius 300,000: 106 against 130 ms): their five-instruction test gains too little here to

@@ -58,10 +58,10 @@ int plane_row_words(int mode) { return mode == kBandShared ? kRowWordsS : kRowWo
 // Per four columns and row a warp issues about 336, 170 or 90 adders for unions of 1, 2 or 4 windows and
 // 90 instructions for each union of its 1,024 x (4 / kUnion) that reaches the threshold (binomial tails of
 // 238 and 272 cells: 8e-4 and 9e-3 at 40, 5e-5 and 1e-3 at 44). Measured, radius 100,000, independent
-// bands, with 1 / 2 / 4: threshold 39 33.5 / 40.0 ms, 40 31.1 / 32.4 / 85.1, 42 28.3 / 25.5 / 44.4, 46 27.6 /
-// 22.6 / 23.4, 47 27.6 / 22.4 / 22.3, 60 27.5 / 22.2 / 20.6; radius 300,000, grouped bands: 38 313 / 432, 40 266 /
-// 240 / 727, 46 216 / 153 / 155, 47 216 / 151 / 145; radius 1,250,000, shared LCG: 46 3,339 / 2,052 / 2,078, 48
-// 3,332 / 2,015 / 1,783.
+// bands, with 1 / 2 / 4: threshold 39 33.6 / 40.1 ms, 40 31.3 / 32.4 / 85.5, 42 28.4 / 25.5 / 44.6, 46 27.7 /
+// 22.5 / 23.6, 47 27.6 / 22.4 / 22.5, 60 27.6 / 22.2 / 20.8; radius 300,000, grouped bands: 38 311 / 434, 40 265 /
+// 241 / 726, 46 216 / 153 / 155, 47 216 / 152 / 145; radius 1,250,000, shared LCG: 46 3,355 / 2,061 / 2,086, 48
+// 3,345 / 2,026 / 1,785.
 constexpr int kUnionTwoFrom = 40, kUnionFourFrom = 47;
 int plane_union(int min_size) { return min_size >= kUnionFourFrom ? 4 : min_size >= kUnionTwoFrom ? 2 : 1; }
 
