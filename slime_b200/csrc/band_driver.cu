@@ -1,6 +1,7 @@
 // band_driver.cu -- host side of the band engine (scan_band.cu) and its redraw correction.
 #include <algorithm>
 #include <chrono>
+#include <cmath>
 #include <thread>
 #include <vector>
 
@@ -273,13 +274,17 @@ bool Context::scan_band(const SearchSpec& q, std::vector<Hit>& best, Counts& h,
             const int32_t nb = (int32_t)std::min<int64_t>(nb_max, nJ - j0);
             if (nb <= 0) break;
             const int64_t tiles = G.tiles;
-            // At most 24 waves a launch, and no more tiles than three quarters of the hit buffer are expected to
-            // take (an upper bound can stop the gate where many sites share a count; a launch that overflows is
-            // run again in halves: radius 450,000, counts 38 to 40 2,273 ms).
+            // At most 24 waves a launch. More sites expected than the hit buffer holds (an upper bound can stop the
+            // gate where many share a count): as many even launches as it takes at four fifths of the buffer each. A
+            // launch that overflows is run again in halves (radius 450,000, counts 38 to 40 2,273 ms, now 1,489);
+            // one more than needed costs a wave (109,888, 41 to 46, 33 ms of kernel and 11 more).
             int64_t chunk = std::max<int64_t>(grid, std::min<int64_t>(tiles, (int64_t)grid * 24));
-            const double sent = (double)W * (double)H * (tail_share(emit_min) - tail_share(q.max_size + 1));
-            if (sent > 0.75 * (double)cap)
-                chunk = std::max<int64_t>(1, std::min<int64_t>(chunk, (int64_t)(0.75 * (double)cap * (double)(ngroups * tiles) / sent)));
+            const double sent = ((double)W * (double)H - 3.14159265358979 * (double)q.rd_min * (double)q.rd_min) *
+                                (tail_share(emit_min) - tail_share(q.max_size + 1)) / (double)ngroups;
+            if (sent > 0.95 * (double)cap) {
+                const int64_t launches = (int64_t)std::ceil(sent / (0.8 * (double)cap));
+                chunk = std::max<int64_t>(1, std::min<int64_t>(chunk, (tiles + launches - 1) / launches));
+            }
             for (int64_t t0 = 0; t0 < tiles;) {
                 while (paused.load() && !cancel.load()) std::this_thread::sleep_for(std::chrono::milliseconds(20));
                 if (cancel.load()) { cancelled = true; return true; }
